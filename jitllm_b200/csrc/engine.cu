@@ -6,6 +6,7 @@
 
 #include <set>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -111,6 +112,7 @@ struct jl_ctx {
     float *gemm_scratch = nullptr;       // split-column partial tiles of the tensor-core path
     size_t gemm_scratch_floats = 0;
     unsigned *gemm_counters = nullptr;   // one arrival counter per output tile, zero between launches
+    void *split_ws = nullptr;            // stand-alone products: one slab of activation rows as binary16 hi / lo parts
     float *part = nullptr;      // row-parallel partial sums before the all-reduce, [row_cap][dim]
     float *best = nullptr;      // local (value, index) of the arg-max and the gathered pairs
     // peer-memory exchange (tp_exchange.cuh): this GPU's inbox, every rank's inbox as mapped here
@@ -198,6 +200,7 @@ int dev_alloc(jl_ctx *ctx, void **p, size_t bytes) {
 // ---- NCCL, bound at run time (the library itself does not link against it) ---------------------
 constexpr int kGemmCounters = 16384;
 constexpr size_t kGemmScratchFloats = size_t(16) << 20;  // 64 MiB
+constexpr size_t kSplitWsBytes = size_t(64) << 20;
 
 struct NcclId {
     char b[128];
@@ -693,6 +696,22 @@ int launch_gemm(jl_ctx *ctx, const DevTensor &w, const float *x, int n, float *y
     return launch_gemm_segs(ctx, ws, ys, rs, 1, x, n, launches, in_kind, presplit);
 }
 
+// The arguments that every tensor-core launch of n rows against matrices like w shares.
+GemmArgs gemm_args(jl_ctx *ctx, const DevTensor &w, int n) {
+    GemmArgs g = {};
+    g.type = w.type;
+    g.cols = int(w.cols);
+    g.n = n;
+    g.status = ctx->d_status;
+    g.scratch = ctx->gemm_scratch;
+    g.scratch_floats = ctx->gemm_scratch_floats;
+    g.counters = ctx->gemm_counters;
+    g.counters_len = kGemmCounters;
+    g.sm_count = ctx->sm_count;
+    g.programmatic = ctx->use_pdl;
+    return g;
+}
+
 // Several matrices of one type against the same rows (Q, K, V; gate, up) in one launch where one kernel takes them
 // all, else one matrix at a time.
 int launch_gemm_segs(jl_ctx *ctx, const DevTensor *const *w, float *const *y, const float *const *res, int nseg,
@@ -728,7 +747,7 @@ int launch_gemm_segs(jl_ctx *ctx, const DevTensor *const *w, float *const *y, co
         }
         return JL_OK;
     }
-    GemmArgs g = {};
+    GemmArgs g = gemm_args(ctx, *w[0], n);
     if (in_kind >= 0 && ctx->xb16 != nullptr && n <= ctx->row_cap) {
         if (!presplit) {  // otherwise the producing kernel already wrote the hi / lo rows
             const int cols = int(w[0]->cols);
@@ -747,20 +766,41 @@ int launch_gemm_segs(jl_ctx *ctx, const DevTensor *const *w, float *const *y, co
         if (!w[s]->has_tmap) return fail(ctx, JL_ERR_UNSUPPORTED, "matrix-matrix product needs a quantised matrix");
         g.seg[s] = {w[s]->data, &w[s]->tmap, y[s], res ? res[s] : nullptr, int(w[s]->rows)};
     }
-    g.type = w[0]->type;
-    g.cols = int(w[0]->cols);
     g.x = x;
-    g.n = n;
-    g.status = ctx->d_status;
-    g.scratch = ctx->gemm_scratch;
-    g.scratch_floats = ctx->gemm_scratch_floats;
-    g.counters = ctx->gemm_counters;
-    g.counters_len = kGemmCounters;
-    g.sm_count = ctx->sm_count;
-    g.programmatic = ctx->use_pdl;
     cudaError_t e = gemm_tc_launch(g, ctx->stream);
     if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "matrix-matrix launch failed: %s", cudaGetErrorString(e));
     ++*launches;
+    return JL_OK;
+}
+
+// A stand-alone product. More rows than one token tile of the in-kernel conversion (64) have their activations split
+// into binary16 parts first, by slabs that fit the workspace: converting them inside the product kernel repeats that
+// work for every 128 weight rows.
+int launch_product(jl_ctx *ctx, const DevTensor &w, const float *x, int n, float *y, uint64_t *launches) {
+    const size_t cols = size_t(w.cols);
+    size_t slab = kSplitWsBytes / (4 * cols) / 256 * 256;
+    const size_t row_tiles = (size_t(w.rows) + 255) / 256;  // two arrival counters per 256 x 256 output tile
+    if (slab > kGemmCounters / 2 / row_tiles * 256) slab = kGemmCounters / 2 / row_tiles * 256;
+    if (n <= 64 || slab < 256) return launch_gemm(ctx, w, x, n, y, nullptr, launches);
+    for (size_t t0 = 0; t0 < size_t(n); t0 += slab) {
+        const int rows = int(std::min(slab, size_t(n) - t0));
+        char *hi = static_cast<char *>(ctx->split_ws), *lo = hi + size_t(rows) * cols * 2;
+        cudaError_t e = split_rows_launch(x + t0 * cols, size_t(rows) * cols, hi, lo, ctx->stream, ctx->use_pdl);
+        if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "activation split launch failed: %s", cudaGetErrorString(e));
+        ++*launches;
+        GemmTensorMap xmap;
+        e = gemm_make_activation_map(&xmap, hi, rows, int64_t(cols), gemm_token_tile(rows));
+        if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "activation descriptor failed: %s", cudaGetErrorString(e));
+        GemmArgs g = gemm_args(ctx, w, rows);
+        g.seg[0] = {w.data, &w.tmap, y + t0 * size_t(w.rows), nullptr, int(w.rows)};
+        g.nseg = 1;
+        g.x = x + t0 * cols;
+        g.xmap = &xmap;
+        g.x_lo_row = rows;
+        e = gemm_tc_launch(g, ctx->stream);
+        if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "matrix-matrix launch failed: %s", cudaGetErrorString(e));
+        ++*launches;
+    }
     return JL_OK;
 }
 
@@ -1152,6 +1192,7 @@ int32_t jl_init(int32_t device_id, jl_ctx **out) {
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->gemm_scratch), kGemmScratchFloats * 4);
     if (e == cudaSuccess) ctx->gemm_scratch_floats = kGemmScratchFloats;
+    if (e == cudaSuccess) e = cudaMalloc(&ctx->split_ws, kSplitWsBytes);
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->gemm_counters), kGemmCounters * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->gemm_counters, 0, kGemmCounters * sizeof(unsigned));
     if (e != cudaSuccess) {
@@ -1175,6 +1216,7 @@ int32_t jl_destroy(jl_ctx *ctx) {
     if (ctx->flush_buf) cudaFree(ctx->flush_buf);
     if (ctx->d_status) cudaFree(ctx->d_status);
     if (ctx->gemm_scratch) cudaFree(ctx->gemm_scratch);
+    if (ctx->split_ws) cudaFree(ctx->split_ws);
     if (ctx->gemm_counters) cudaFree(ctx->gemm_counters);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -2083,8 +2125,8 @@ int32_t jl_gemv_dev(jl_ctx *ctx, const jl_tensor *w, const float *x_dev, int32_t
     uint64_t launches = 0;
     static const int gemm_min_n = [] { const char *v = getenv("JITLLM_B200_GEMM_MIN_N"); return v ? atoi(v) : 8; }();
     if (n >= gemm_min_n && w->t.has_tmap) {
-        // Wide enough for the tensor cores: one tcgen05 matrix-matrix launch.
-        int rc = launch_gemm(ctx, w->t, x_dev, n, y_dev, nullptr, &launches);
+        // Wide enough for the tensor cores.
+        int rc = launch_product(ctx, w->t, x_dev, n, y_dev, &launches);
         ctx->counters.kernel_launches += launches;
         return rc;
     }

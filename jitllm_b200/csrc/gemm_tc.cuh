@@ -51,6 +51,11 @@ struct GemmArgs {
 // Sets the shared-memory attribute of every instantiation (call once, outside stream capture).
 cudaError_t gemm_tc_configure();
 cudaError_t gemm_tc_launch(const GemmArgs &args, cudaStream_t stream);
+// The CTA-pair kernel behind gemm_tc_launch for more than kGemmNarrowRows rows of pre-split activations; the
+// activation map is the one for 128-row boxes.
+constexpr int kGemmNarrowRows = 128;
+cudaError_t gemm_wide_configure();
+cudaError_t gemm_wide_launch(const GemmArgs &args, cudaStream_t stream);
 cudaError_t gemm_trace_bind(unsigned long long *buf, unsigned cap, int mode);
 
 }  // namespace jl

@@ -89,3 +89,25 @@ def test_widest_sweep_batch(dev, oracle, t):
     err = rel_l2(got[sample], want)
     assert err < BAR and err < EXPECT, err
     assert np.all(np.isfinite(got))
+
+
+@pytest.mark.parametrize("t", FORMATS + [GGMLType.Q4_1, GGMLType.Q5_K, GGMLType.Q6_K])
+@pytest.mark.parametrize("rows,cols,n", [(100, 256, 129),     # one tile, half of it (and most of the token half) empty
+                                         (256, 512, 256),     # exactly one tile
+                                         (300, 2048, 257),    # a second row tile and a second token tile of one row
+                                         (1536, 4096, 470),   # 12 tiles on 74 CTA pairs: several pairs per tile
+                                         (6144, 1024, 513),   # 72 tiles: ranges aligned to tiles
+                                         (12900, 512, 300)])  # 102 tiles: ranges end inside tiles
+def test_wide_products_on_cta_pairs(dev, oracle, t, rows, cols, n):
+    """More than 128 rows: 256 x 256 tiles on CTA pairs. Same operands as the narrow kernel (weights rounded once to
+    binary16, 2^-12 relative on average; activations in 22 bits), so the same expected error."""
+    make = jl.synth_tensor if t in FORMATS else jl.random_blocks
+    w = make(t, rows * cols, seed=rows + cols + n)
+    x = np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)
+    got = dev.matmul(t, w, rows, cols, x)
+    sample = sorted({0, 1, 127, 128, 255, 256, n // 2, n - 2, n - 1} & set(range(n)))
+    want = oracle.matmul(int(t), w, x[sample], rows, cols)
+    err = np.linalg.norm(got[sample] - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() < EXPECT, err
+    assert np.all(np.isfinite(got))
+    assert np.array_equal(dev.matmul(t, w, rows, cols, x), got)  # partial tiles are added in a fixed order
