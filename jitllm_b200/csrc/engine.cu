@@ -866,6 +866,7 @@ int enqueue_rows_step(jl_ctx *ctx, int n, bool with_logits, bool advance, uint64
             a.append = own_sequences ? 1 : 0;
             a.partial = ctx->att_partial;
             a.counters = ctx->att_count;
+            a.status = ctx->d_status;
             if (attn_presplit) {  // the output projection reads these rows as binary16 hi / lo parts
                 a.out_hi = ctx->xb16;
                 a.out_lo = static_cast<char *>(ctx->xb16) + size_t(ctx->row_cap) * ctx->l_qdim * 2;
@@ -1188,6 +1189,7 @@ int32_t jl_init(int32_t device_id, jl_ctx **out) {
     if (e == cudaSuccess) e = gemv_configure();
     if (e == cudaSuccess) e = attention_configure();
     if (e == cudaSuccess) e = gemm_tc_configure();
+    if (e == cudaSuccess) e = attention_prompt_configure();
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->d_status), sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->gemm_scratch), kGemmScratchFloats * 4);

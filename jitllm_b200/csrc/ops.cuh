@@ -30,12 +30,15 @@ struct AttnArgs {
     int append;  // 1: the CTA owning the new position rotates k and appends k,v; 0: pages already hold it
     float *partial;     // scratch [width][heads][nsplit][head_dim + 2]
     unsigned *counters; // scratch [width][kv_heads], zero between launches
+    int *status;        // device status word (attention_prompt_launch), nullable
 };
 
 cudaError_t attention_configure();
 cudaError_t attention_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic);
-// The rows of one prompt chunk (all of one sequence, their keys already in the pages; append = 0): tiles of
-// query rows against tiles of keys on the tensor cores instead of one walk over the pages per row.
+// The rows of one prompt chunk (all of one sequence, their keys already in the pages; append = 0): tiles of 128 rows
+// (heads x tokens) against tiles of 128 keys on the tensor cores (attn_prompt_tc.cu) instead of one walk over the
+// pages per row.
+cudaError_t attention_prompt_configure();
 cudaError_t attention_prompt_launch(const AttnArgs &a, int n, cudaStream_t stream, bool programmatic);
 // A decode batch of at least four rows (one sequence per row, append = 1): one CTA per (row, KV head) with the
 // query heads as the rows of a tensor-core tile; rotates and appends the step's own key and value itself.

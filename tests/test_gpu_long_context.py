@@ -120,6 +120,38 @@ def test_prompt_tiles_ragged_and_continued(dev, oracle, heads, kv_heads, head):
     kv.close()
 
 
+@pytest.mark.parametrize("heads,kv_heads,head,page,chunks", [(4, 1, 128, 16, (127, 9)),      # the last key tile is full, then one key more
+                                                             (4, 2, 128, 24, (128, 129)),    # pages that do not divide a key tile
+                                                             (2, 2, 64, 16, (255, 8)),       # 128 rows of one head in a CTA
+                                                             (8, 1, 128, 7, (8, 33, 215))])  # 16 rows a CTA, tiny odd pages
+def test_prompt_attention_at_tile_edges(dev, oracle, heads, kv_heads, head, page, chunks):
+    """Prompts whose chunks end at, just before and just behind the 128-key tiles, with page sizes that do and do not
+    divide them; checked through the logits of the tokens that follow, which read every key and value."""
+    cfg = _config(heads=heads, kv_heads=kv_heads, head=head, ctx=384)
+    tensors = jl.synth_model_tensors(cfg, GGMLType.Q8_0, seed=33, std=0.05)
+    om = oracle.Model(cfg, tensors)
+    model = jl.load_model(dev, cfg, tensors, *om.rope_tables())
+    bps = -(-cfg.contextLength // page)
+    kv = model.createKvStorage(jl.KvStorageRequest(bps, bps, 1, page, cfg.numberOfLayers, cfg.kvDim))
+    kv.publishBlockTable(np.random.default_rng(5).permutation(bps).astype(np.int32))
+    kv.fill(0x7E00)
+    total, steps = sum(chunks), 3
+    toks = np.random.default_rng(6).integers(0, cfg.vocabularySize, size=total + steps)
+    bound = jl.B200InvocationBoundary(model, kvSlot=0)
+    at = 0
+    for n in chunks:
+        bound.prefill([int(v) for v in toks[at:at + n]], at)
+        at += n
+    for pos in range(total):
+        om.forward_no_logits(int(toks[pos]), pos)
+    for pos in range(total, total + steps):
+        want = om.forward(int(toks[pos]), pos)
+        got = bound.invoke(int(toks[pos]), pos)
+        assert np.all(np.isfinite(got.logits)), pos
+        assert float(np.max(np.abs(got.logits - want))) < LOGIT_BAR
+    kv.close()
+
+
 @pytest.mark.parametrize("heads,kv_heads,head", [(8, 2, 64), (4, 1, 128), (2, 2, 128), (8, 1, 64)])
 def test_batch_attention_kernel_on_ragged_batches(oracle, monkeypatch, heads, kv_heads, head):
     """The tensor-core decode attention for wide batches (one CTA per row and KV head, query heads as the rows
