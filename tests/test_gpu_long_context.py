@@ -122,7 +122,7 @@ def test_prompt_tiles_ragged_and_continued(dev, oracle, heads, kv_heads, head):
 
 @pytest.mark.parametrize("heads,kv_heads,head,page,chunks", [(4, 1, 128, 16, (127, 9)),      # the last key tile is full, then one key more
                                                              (4, 2, 128, 24, (128, 129)),    # pages that do not divide a key tile
-                                                             (2, 2, 64, 16, (255, 8)),       # 128 rows of one head in a CTA
+                                                             (4, 4, 64, 16, (255, 8)),       # 128 rows of one head in a CTA
                                                              (8, 1, 128, 7, (8, 33, 215))])  # 16 rows a CTA, tiny odd pages
 def test_prompt_attention_at_tile_edges(dev, oracle, heads, kv_heads, head, page, chunks):
     """Prompts whose chunks end at, just before and just behind the 128-key tiles, with page sizes that do and do not
