@@ -96,7 +96,6 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
     volatile uint32_t *abort_flag = tmem_ptr + 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int kvh = blockIdx.y, cta_row0 = blockIdx.x * RQ;
-    pdl_launch_dependents();
 
     if (warp == 12) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)), "r"(kPtCols)
@@ -139,6 +138,9 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_ptr;
+    // Only now: a dependent kernel's CTA that came to this SM ahead of the allocation could take the tensor memory and then
+    // wait for this grid, which would wait for it.
+    pdl_launch_dependents();
     bool ok = true;
 
     if (warp == 12) {

@@ -1,0 +1,45 @@
+"""Rules that a run cannot show to be kept (a kernel that breaks one may still pass every numerics test, until another
+kernel lands beside it on an SM), checked on the text of the kernels."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "jitllm_b200" / "csrc"
+
+
+def _code(path):
+    """The source without comments, line breaks kept."""
+    text = re.sub(r"/\*.*?\*/", lambda m: "\n" * m.group().count("\n"), path.read_text(), flags=re.S)
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _function_at(text, start):
+    """The body of the function whose definition starts at `start`."""
+    open_at = text.index("{", start)
+    depth = 0
+    for i in range(open_at, len(text)):
+        depth += {"{": 1, "}": -1}.get(text[i], 0)
+        if depth == 0:
+            return text[open_at:i + 1]
+    raise AssertionError("unbalanced braces")
+
+
+def _tensor_memory_kernels():
+    for path in sorted(CSRC.glob("*.cu")):
+        text = _code(path)
+        for m in re.finditer(r"__global__", text):
+            body = _function_at(text, m.start())
+            if "tmem_alloc(" in body or "tcgen05.alloc" in body:
+                name = re.search(r"(\w+_kernel)\s*\(", text[m.start():]).group(1)
+                yield pytest.param(body, id=f"{path.name}:{name}")
+
+
+@pytest.mark.parametrize("body", _tensor_memory_kernels())
+def test_dependents_are_released_after_the_tensor_memory_is_allocated(body):
+    """A dependent kernel's CTA that lands on the SM of a CTA which has not allocated yet could take the tensor memory and
+    then wait for that CTA's grid to finish: neither would ever go on."""
+    alloc = re.search(r"tmem_alloc\(|tcgen05\.alloc", body).start()
+    barrier = body.index("__syncthreads()", alloc)  # the allocating warp has passed it with its columns
+    release = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", body)]
+    assert release and min(release) > barrier
