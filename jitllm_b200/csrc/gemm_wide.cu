@@ -2,13 +2,17 @@
 // products): Y[n][rows] = X[n][cols] . W[rows][cols]^T on CTA pairs, same operands as gemm_tc.cu (weights rounded
 // once to binary16 by the same code, activations as binary16 hi + lo parts, binary32 accumulation).
 //
-// What bounds it: the tensor cores. A 128 x 256 block of weights takes about 1400 issue cycles to convert; against
-// 128 tokens the tensor core needs 2048 cycles for it (hi and lo parts), so the two are nearly level and every
-// hand-over shows, against 256 tokens 4096. The tile is therefore 256 weight rows x 256 tokens on two SMs
-// (cta_group::2, M = 256, N = 256): each CTA converts its own 128 rows into its own tensor memory and stages one half
-// of the tokens, which both tensor cores read, so an SM fetches 32 KB of activations per 1024 tensor cycles instead
-// of 64 KB. The hi and the lo product go into one accumulator (256 of the 512 tensor-memory columns; the other 256
-// hold eight operand stages of 64 K elements).
+// What bounds it: the tensor cores and the conversion, nearly level. The tile is 256 weight rows x 256 tokens on two SMs
+// (cta_group::2, M = 256, N = 256): each CTA converts its own 128 rows into its own tensor memory and stages one half of
+// the tokens, which both tensor cores read. The accumulator takes 256 of the 512 tensor-memory columns; the other 256 hold
+// eight operand stages of 64 K elements.
+//
+// A pair walks its part of a tile twice: first against the lo parts of the activations, then against the hi parts, into
+// one accumulator. The tensor core cuts every addition off at the accumulator's last place, so the lo products (2^-11 of
+// the hi ones) have to be summed before the hi sum is there: side by side in one pass, a product of 4096 columns was
+// 9.2e-6 from the 64-bit sum (2-norm, weights that binary16 holds exactly), in two passes it is 4.4e-6, as with an
+// accumulator for either part (gemm_tc.cu). The weights are converted twice for it, which costs a tenth (14336 x 4096
+// against 512 rows 99 -> 110 us). Two accumulators leave room for 192 tokens and half the operand stages: 130 us.
 //
 // One persistent CTA pair per two SMs; the work list (256-row tile, 256-token tile, 256-column raw stage) is cut
 // into equal ranges, one per pair, as in gemm_tc.cu. Roles in a CTA, meeting only at mbarriers:
@@ -22,11 +26,12 @@
 //     first CTA's barrier.
 // Every wait is bounded; a wait that runs out sets the status word and the CTA winds down.
 //
-// Measured (B200, 14336 x 4096 against 512 rows): Q4_K 277 us -> 112 us with the splitting of the activations (the
-// 64-token kernel converted weights and activations again for every tile), Q8_0 101 us; four layers of the 8B shapes
-// against 512 rows: 2.21 -> 1.91 ms; an 8B Q4_K prompt of 471 tokens 19.9 -> 17.0 ms. Folding the
-// partial tiles out of memory alone, by the epilogue's warps, took 15-19 us of a launch; keeping the last arriver's
-// share in tensor memory and lending it the idle conversion warps brought a 4096 x 4096 product from 55 to 41 us.
+// Measured (B200, device time of a stand-alone product with the splitting of its activations, cold L2) against the
+// 64-token kernel, which converted weights and activations again for every tile: 14336 x 4096 against 512 rows Q4_K
+// 262 -> 110 us, Q8_0 268 -> 112; against 140 rows 115 -> 64, against 2048 985 -> 380; Q8_0 4096 x 4096 against 512 rows
+// 98 -> 50. The partial tiles folded out of memory alone, by the epilogue's warps, took 15-19 us of a launch; keeping the
+// last arriver's share in tensor memory and lending it the idle conversion warps brought a 4096 x 4096 product from 55 to
+// 41 us (one pass, activations split before).
 #include "gemm_tc_core.cuh"
 
 #include <cstring>
@@ -47,9 +52,8 @@ static_assert(kAccCols + kAStages * kAStageCols == kWideTmemCols, "tensor memory
 
 template <int TYPE>
 struct WideSmem {
-    static constexpr int b_half = kHalfN * kUnitK * 2;  // hi (or lo) part of this CTA's tokens
-    static constexpr int b_stage = 2 * b_half;
-    static constexpr int b_stages = 4;
+    static constexpr int b_stage = kHalfN * kUnitK * 2;  // hi or lo part of this CTA's tokens
+    static constexpr int b_stages = 8;                  // at most kAStages: an operand stage handed back frees one
     static constexpr int bar_bytes = 512;
     static constexpr int raw_stage = RawFmt<TYPE>::stage_bytes;
     static constexpr int raw_fit = (227 * 1024 - 1024 - bar_bytes - b_stages * b_stage) / raw_stage;
@@ -102,11 +106,10 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
         ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(leader_bar)
         : "memory");
 }
-// The MMAs of one operand stage (four K = 16 steps, hi then lo part of the activations, one accumulator) and the
-// commit that hands the stage back to both CTAs; issued by one elected lane of a converged warp.
+// The MMAs of one operand stage (four K = 16 steps) and the commit that hands the stage back to both CTAs; issued by one
+// elected lane of a converged warp.
 __device__ __forceinline__ void umma_stage_pair(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,
                                                 uint32_t done_bar, uint32_t accumulate_first) {
-    constexpr int kLo = WideSmem<kQ4_K>::b_half >> 4;  // descriptor step from the hi rows to the lo rows
     asm volatile(
         "{\n\t"
         ".reg .pred pe, pacc, pone;\n\t"
@@ -119,24 +122,15 @@ __device__ __forceinline__ void umma_stage_pair(uint32_t d_tmem, uint32_t a_tmem
         "mov.b16 mask, 3;\n\t"
         "mov.b64 bd, {%2, %3};\n\t"
         "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], bd, %4, pacc;\n\t"
-        "add.u32 lo, %2, %7;\n\t mov.b64 bd, {lo, %3};\n\t"
-        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], bd, %4, pone;\n\t"
         "add.u32 ac, %1, 8;\n\t add.u32 lo, %2, 2;\n\t mov.b64 bd, {lo, %3};\n\t"
-        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
-        "add.u32 lo, %2, %8;\n\t mov.b64 bd, {lo, %3};\n\t"
         "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
         "add.u32 ac, %1, 16;\n\t add.u32 lo, %2, 4;\n\t mov.b64 bd, {lo, %3};\n\t"
         "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
-        "add.u32 lo, %2, %9;\n\t mov.b64 bd, {lo, %3};\n\t"
-        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
         "add.u32 ac, %1, 24;\n\t add.u32 lo, %2, 6;\n\t mov.b64 bd, {lo, %3};\n\t"
-        "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
-        "add.u32 lo, %2, %10;\n\t mov.b64 bd, {lo, %3};\n\t"
         "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], [ac], bd, %4, pone;\n\t"
         "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%5], mask;\n\t"
         "}"
-        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(done_bar), "r"(accumulate_first), "n"(kLo),
-          "n"(kLo + 2), "n"(kLo + 4), "n"(kLo + 6)
+        ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(done_bar), "r"(accumulate_first)
         : "memory");
 }
 __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
@@ -228,6 +222,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     uint64_t *acc_empty = acc_full + 1;    // first CTA: accumulator read out by both CTAs
     uint64_t *epi_bar = acc_empty + 1;     // the epilogue warps' own barrier
     uint64_t *last_fold = epi_bar + 1;     // it is known whether the range's last tile is finished here
+    static_assert(BS <= AS, "activation stages");
     static_assert((2 * AS + BS + 2 * 4 + 4) * 8 + 80 <= S::bar_bytes, "barrier block");
     uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(base + S::bar_off + S::bar_bytes - 16);
     volatile uint32_t *fold_flags = reinterpret_cast<uint32_t *>(base + S::bar_off + S::bar_bytes - 64);  // four, taken in turn
@@ -237,7 +232,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     int tiles = 0;
     for (int s = 0; s < a.nseg; ++s) tiles += (a.seg[s].rows + kPairM - 1) / kPairM;
     const int n_tiles = (a.n + kWideN - 1) / kWideN;
-    const int raw_total = a.cols / kRawK;
+    const int raw_total = a.cols / kRawK;  // the second pass over them is not counted
     const int total = tiles * n_tiles * raw_total;
     const int pairs = int(gridDim.x >> 1), pair = int(blockIdx.x >> 1);
     const int lo = range_lo(total, pair, pairs), hi = range_lo(total, pair + 1, pairs);
@@ -303,47 +298,51 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     bool ok = true;
 
     if (warp == kEpiWarps + kConvWarps + 1) {
-        // ---- raw weight stages: this CTA's 128 rows (past the end of the matrix: zeros) -------------------
+        // ---- raw weight stages, twice a tile: this CTA's 128 rows (past the end of the matrix: zeros) -----
         if (lane == 0) {
             const uint64_t policy = policy_evict_first();
             fence_proxy_async();
-            int i = 0, cur_u = -1;
-            TileRef tr = {0, 0};
-            for (int f = lo; f < hi && *abort_flag == 0u; ++f, ++i) {
-                const int u = f / raw_total, r = f - u * raw_total;
-                if (u != cur_u) {
-                    cur_u = u;
-                    tr = locate(u / n_tiles);
-                }
-                const int st = i % RS;
-                if (i >= RS && !(ok = mbar_poll_bounded(raw_empty + st, uint32_t(i / RS - 1) & 1u))) break;
-                mbar_expect_tx(raw_full + st, R::stage_bytes);
+            int i = 0;
+            for (int f = lo, seg_end; f < hi && ok && *abort_flag == 0u; f = seg_end) {
+                const int u = f / raw_total;
+                seg_end = min((u + 1) * raw_total, hi);
+                const TileRef tr = locate(u / n_tiles);
                 const CUtensorMap *tmap = tr.seg == 0 ? &tm0 : (tr.seg == 1 ? &tm1 : &tm2);
-                if (n_tiles == 1)  // read once; otherwise the next token tiles find the stage in L2
-                    tma_load_2d(base + S::raw_off + st * R::stage_bytes, tmap, r * (R::row_bytes / 4), tr.row0, raw_full + st,
-                                policy);
-                else
-                    tma_load_2d_plain(base + S::raw_off + st * R::stage_bytes, tmap, r * (R::row_bytes / 4), tr.row0,
-                                      raw_full + st);
+                const int len = seg_end - f;
+                for (int k = 0; k < 2 * len && *abort_flag == 0u; ++k, ++i) {
+                    const int r = f + (k < len ? k : k - len) - u * raw_total;
+                    const int st = i % RS;
+                    if (i >= RS && !(ok = mbar_poll_bounded(raw_empty + st, uint32_t(i / RS - 1) & 1u))) break;
+                    mbar_expect_tx(raw_full + st, R::stage_bytes);
+                    if (n_tiles == 1 && k >= len)  // read for the last time; otherwise the next reader finds the stage in L2
+                        tma_load_2d(base + S::raw_off + st * R::stage_bytes, tmap, r * (R::row_bytes / 4), tr.row0, raw_full + st,
+                                    policy);
+                    else
+                        tma_load_2d_plain(base + S::raw_off + st * R::stage_bytes, tmap, r * (R::row_bytes / 4), tr.row0,
+                                          raw_full + st);
+                }
             }
             if (!ok || *abort_flag != 0u)  // winding down: no copy may still be on its way into this CTA
                 for (int k = i > RS ? i - RS : 0; k < i; ++k) mbar_poll_bounded(raw_full + k % RS, uint32_t(k / RS) & 1u);
         }
     } else if (warp == kEpiWarps + kConvWarps + 2) {
-        // ---- activation rows: this CTA's 128 tokens of the tile, hi and lo ---------------------------------
+        // ---- activation rows: this CTA's 128 tokens of the tile, the lo parts, then the hi parts ------------
         if (lane == 0) {
             pdl_wait();
-            const int stages = (hi - lo) * 4;
+            const int stages = (hi - lo) * 8;
             int q = 0;
-            for (; q < stages && *abort_flag == 0u; ++q) {
-                const int f = lo + (q >> 2), u = f / raw_total, r = f - u * raw_total;
-                const int k0 = r * kRawK + (q & 3) * kUnitK, tok = (u % n_tiles) * kWideN + int(rank) * kHalfN;
-                const int s = q % BS;
-                if (q >= BS && !(ok = mbar_poll_bounded(done + (q - BS) % AS, uint32_t((q - BS) / AS) & 1u))) break;
-                if (rank == 0) mbar_expect_tx(b_full + s, 2 * S::b_stage);
-                const uint32_t dst = smem_u32(base + s * S::b_stage), bar = leader_addr(smem_u32(b_full + s));
-                tma_load_2d_pair(dst, &tmx, k0, tok, bar);
-                tma_load_2d_pair(dst + S::b_half, &tmx, k0, a.x_lo_row + tok, bar);
+            for (int f = lo, seg_end; f < hi && ok && *abort_flag == 0u; f = seg_end) {
+                const int u = f / raw_total;
+                seg_end = min((u + 1) * raw_total, hi);
+                const int tok = (u % n_tiles) * kWideN + int(rank) * kHalfN, k_lo = (f - u * raw_total) * kRawK;
+                const int len = 4 * (seg_end - f);
+                for (int k = 0; k < 2 * len && *abort_flag == 0u; ++k, ++q) {  // the lo parts of the tile's range, then the hi parts
+                    const int s = q % BS;
+                    if (q >= BS && !(ok = mbar_poll_bounded(done + (q - BS) % AS, uint32_t((q - BS) / AS) & 1u))) break;
+                    if (rank == 0) mbar_expect_tx(b_full + s, 2 * S::b_stage);
+                    tma_load_2d_pair(smem_u32(base + s * S::b_stage), &tmx, k_lo + (k < len ? k : k - len) * kUnitK,
+                                     (k < len ? a.x_lo_row : 0) + tok, leader_addr(smem_u32(b_full + s)));
+                }
             }
             if (!ok || *abort_flag != 0u) {
                 if (rank == 0)
@@ -367,7 +366,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             while (f < hi && ok && *abort_flag == 0u) {
                 const int u_hi = (f / raw_total + 1) * raw_total;
                 const int seg_end = u_hi < hi ? u_hi : hi;
-                const int nstage = 4 * (seg_end - f);
+                const int nstage = 8 * (seg_end - f);
                 if (turn > 0) ok = wait_pair(smem_u32(acc_empty), uint32_t(turn - 1) & 1u);
                 for (int k = 0; k < nstage && ok; ++k) {
                     ok = wait_pair(a_full0 + 8u * uint32_t(sa), pa) && wait_pair(b_full0 + 8u * uint32_t(sb), pb);
@@ -417,7 +416,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         int s = grp, rev = 0, st = 0, unit = grp;
         uint32_t raw_par = 0;
         static_assert(kConvGroups <= 4 && kConvGroups <= AS, "running indices advance by less than a raw stage");
-        const int stages = (hi - lo) * 4;
+        const int stages = (hi - lo) * 8;
         for (int q = grp; q < stages && *abort_flag == 0u; q += kConvGroups) {
             ok = mbar_poll_bounded_u32(raw_full0 + 8u * uint32_t(st), raw_par);
             if (ok && rev > 0) ok = mbar_poll_bounded_u32(done0 + 8u * uint32_t(s), uint32_t(rev - 1) & 1u);

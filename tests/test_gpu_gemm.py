@@ -111,3 +111,25 @@ def test_wide_products_on_cta_pairs(dev, oracle, t, rows, cols, n):
     assert err.max() < EXPECT, err
     assert np.all(np.isfinite(got))
     assert np.array_equal(dev.matmul(t, w, rows, cols, x), got)  # partial tiles are added in a fixed order
+
+
+def test_wide_product_is_as_close_to_64_bits_as_the_narrow_one(dev):
+    """The same rows through the 128-row kernel (an accumulator for either part of the activations) and, as part of a
+    wider block, through the CTA pairs. The weights are whole multiples of 2^-7, exact in binary16, so what is left is the
+    activations' 22 bits and the binary32 sums: 256 steps over 4096 columns that are cut off at the accumulator's last
+    place, 256 * 2^-24 = 1.5e-5 at most. 148 row tiles of 128 and 74 of 256: every sum runs over whole rows in both."""
+    rows, cols, n = 148 * 128, 4096, 256
+    rng = np.random.default_rng(3)
+    q = rng.integers(-127, 128, size=(rows, cols)).astype(np.int8)
+    blocks = np.empty((rows, cols // 32, 34), np.uint8)
+    blocks[:, :, :2] = np.frombuffer(np.float16(2.0 ** -7).tobytes(), np.uint8)
+    blocks[:, :, 2:] = q.reshape(rows, cols // 32, 32).view(np.uint8)
+    x = rng.standard_normal((n, cols)).astype(np.float32)
+    pick = np.sort(rng.choice(rows, 256, replace=False))
+    want = x.astype(np.float64) @ (q[pick].astype(np.float64) * 2.0 ** -7).T
+    err = {}
+    for m in (128, n):
+        got = dev.matmul(GGMLType.Q8_0, blocks.reshape(-1), rows, cols, x[:m])[:, pick]
+        err[m] = np.linalg.norm(got[:128] - want[:128]) / np.linalg.norm(want[:128])
+    assert err[n] < 256 * 2.0 ** -24, err
+    assert err[n] <= 1.05 * err[128], err
