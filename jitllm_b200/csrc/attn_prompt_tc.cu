@@ -5,19 +5,20 @@
 // backend/tornado/layers/TensorCoreBatchAttention.java:227-366, not its code).
 //
 // A CTA takes 128 / G query rows and the G query heads of one KV head: 128 rows that share every key. Per tile of 128
-// keys: S = Qhi K^T + Qlo K^T (both operands in shared memory, 128-byte swizzle, S in tensor memory, two buffers),
+// keys: S = Qlo K^T + Qhi K^T (both operands in shared memory, 128-byte swizzle, S in tensor memory, two buffers),
 // softmax by 256 threads (a row per lane, two threads per row), P as binary16 back into tensor memory, O = P V with V as
 // it lies in the pages (the B operand is "MN-major", so nothing is transposed), and the tile's O is added to registers
 // scaled by the running maximum. The scores of tile t + 1 and the values of tile t - 1 are multiplied while the softmax
 // of tile t runs.
 //
-// Measured (B200, 8B shapes, 512 rows): 373 -> 293 us against 8192 keys, 69 -> 38 us against the first 512; the kernel
-// before it multiplied with mma.sync from registers, read its rows' positions one after the other and stored two bytes at
-// a time. 8B Q8_0 prompt of 8192 tokens 408 -> 306 ms, 8B Q4_K prompt of 471 tokens 17.0 -> 16.4 ms, 1B prompt of 23
-// tokens 1.99 -> 1.95 ms: faster over the whole range, so there is one kernel. What bounds it: 4.3 us per 128 keys against
-// 0.8 us of tensor work and about 1.1 us of exponentials. Without copies after the second tile the 8192-token prompt is 7 %
-// faster, without the exponentials 16 %: the softmax warps' chain (two passes over the scores, two row barriers, adding
-// the tile's O) comes first, then the copies.
+// Measured (B200, one launch of 512 rows at the 8B shapes, cold L2) against the kernel before it, which multiplied with
+// mma.sync from registers, read its rows' positions one after the other and stored two bytes at a time: 73 -> 42 us against
+// the first 512 keys, 204 -> 92 us against 2048, 725 -> 293 us against 8192. Faster over the whole range, so there is one
+// kernel. Distance from a 64-bit softmax (2-norm; standard deviation of the scores 1 to 12, common offset 0 to 2000, 512 to
+// 8192 keys): 3.4e-5 to 2.0e-4, what the rounding of the probabilities leaves, and no more than that kernel's.
+// What bounds it: 4.3 us per 128 keys against 0.8 us of tensor work and about 1.1 us of exponentials. Without copies after
+// the second tile the 8192-token prompt was 7 % faster, without the exponentials 16 %: the softmax warps' chain (two passes
+// over the scores, two row barriers, adding the tile's O) comes first, then the copies.
 // Roles: warps 0-7 softmax and output, warps 8-9 copy keys, 10-11 values (cp.async, a ring of two tiles each), warp 12
 // issues the MMAs. They meet at mbarriers; every wait is bounded and a wait that runs out sets the status word.
 #include "gemm_tc_core.cuh"
@@ -160,12 +161,14 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
                         break;
                     }
                     tc_fence_after();
+                    // The lo part first: every addition is cut off at the accumulator's last place, and the lo products
+                    // (2^-11 of the hi ones) lose nothing that counts while the hi sum is not there yet.
 #pragma unroll
                     for (int part = 0; part < 2; ++part) {
 #pragma unroll
                         for (int k = 0; k < HD / 16; ++k) {
                             const uint32_t off = uint32_t(k >> 2) * S::atom + uint32_t(k & 3) * 32u;
-                            umma_ss(tmem + kPtS + uint32_t(b) * kPtKeys, pt_desc(q0 + uint32_t(part) * S::tile + off, 16),
+                            umma_ss(tmem + kPtS + uint32_t(b) * kPtKeys, pt_desc(q0 + uint32_t(1 - part) * S::tile + off, 16),
                                     pt_desc(k0 + uint32_t(b) * S::tile + off, 16), idesc_s, part + k > 0 ? 1u : 0u);
                         }
                     }
@@ -294,8 +297,10 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
 #pragma unroll
         for (int d = 0; d < kDims; ++d) o[d] = 0.f;
         float m = -INFINITY, l = 0.f, corr = 1.0f;  // corr: what the sums before the tile in flight are scaled by
-        // exp(s / sqrt(HD) - max) = 2^(s * scale - max * scale): one fused multiply-add and one ex2 per score (relative error
-        // 2^-22 before the probability is rounded to binary16, 2^-11)
+        // exp(s / sqrt(HD) - max) = 2^(s * scale - sub), sub = max * scale rounded: one fused multiply-add and one ex2 per score.
+        // Its relative error is 2^-22 of the ex2 and up to |sub| 2^-25 of the rounding of sub. The latter is common to all
+        // keys and leaves with the division, because the sums of earlier tiles are moved from one rounded sub to the next.
+        float sub = 0.f;
         const float scale = 1.4426950408889634f / sqrtf(static_cast<float>(HD));
         const uint32_t lanes = uint32_t((warp & 3) * 32) << 16;
         // the two warps that share these 32 rows
@@ -341,10 +346,11 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
             xch[half * kPtRows + r] = mx;
             row_sync();
             const float mn = fmaxf(m, fmaxf(mx, xch[(half ^ 1) * kPtRows + r]));
-            const float next_corr = (mn == -INFINITY) ? 1.0f : pt_exp2((m - mn) * scale);  // 2^-inf = 0 on the first tile
+            const float next_sub = mn == -INFINITY ? 0.f : mn * scale;  // -inf: nothing but masked keys so far
+            const float next_corr = m == -INFINITY ? 0.f : pt_exp2(sub - next_sub);  // before the first key the sums are 0
             m = mn;
+            sub = next_sub;
             l *= next_corr;
-            const float sub = mn == -INFINITY ? 0.f : mn * scale;  // -inf: nothing but masked keys so far
             uint32_t p[32];
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -359,9 +365,11 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
 #pragma unroll
                 for (int j = 0; j < 16; j += 2) {
                     const float p0 = pt_exp2(fmaf(v[j], scale, -sub)), p1 = pt_exp2(fmaf(v[j + 1], scale, -sub));
-                    sum4[j & 2] += p0;
-                    sum4[(j & 2) + 1] += p1;
-                    p[(g * 16 + j) / 2] = h2_bits(__floats2half2_rn(p0, p1));
+                    const __half2 ph = __floats2half2_rn(p0, p1);
+                    const float2 pr = __half22float2(ph);  // the sum is over what the values are multiplied by
+                    sum4[j & 2] += pr.x;
+                    sum4[(j & 2) + 1] += pr.y;
+                    p[(g * 16 + j) / 2] = h2_bits(ph);
                 }
             }
             l += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);

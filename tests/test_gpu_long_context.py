@@ -197,3 +197,29 @@ def test_batch_attention_kernel_on_ragged_batches(oracle, monkeypatch, heads, kv
                 assert float(np.max(np.abs(got_k - want_k))) <= 4e-3 * float(np.max(np.abs(want_k))), (step, b)
                 positions[b] += 1
         kv.close()
+
+
+@pytest.mark.parametrize("heads,kv_heads,head", [(8, 2, 64), (4, 1, 128)])
+def test_prompt_attention_weights_sum_to_one(dev, oracle, heads, kv_heads, head):
+    """A prompt of one token over and over: every position has the same values, so whatever the weights are, attention
+    returns those values, and the second layer's values are the same at every position as at the first, which has one key
+    and weight 1. What attention may add is the rounding of its binary32 sums, some 1e-7; the pages hold binary16, whose
+    steps are 5e-4 to 1e-3 of a value, so about one element in a thousand may fall on the other side of a rounding. Weights
+    that do not sum to one to that accuracy (rounded probabilities over the sum of the unrounded ones: 1e-5 to 1e-4) show
+    as a quarter of the elements."""
+    cfg = _config(heads=heads, kv_heads=kv_heads, head=head, ctx=256)
+    tensors = jl.synth_model_tensors(cfg, GGMLType.Q8_0, seed=41, std=0.2)
+    model = jl.load_model(dev, cfg, tensors, *oracle.Model(cfg, tensors).rope_tables())
+    bps = cfg.contextLength // 16
+    kv = model.createKvStorage(jl.KvStorageRequest(bps, bps, 1, 16, cfg.numberOfLayers, cfg.kvDim))
+    kv.publishBlockTable(np.arange(bps, dtype=np.int32))
+    kv.fill(0x7E00)
+    P = 200
+    jl.B200InvocationBoundary(model, kvSlot=0).prefill([7] * P, 0)
+    first = [kv.readRow("v", 0, layer, 0) for layer in range(2)]
+    differ = []
+    for pos in range(1, P):
+        assert np.array_equal(kv.readRow("v", 0, 0, pos), first[0]), pos
+        differ.append(np.mean(kv.readRow("v", 0, 1, pos) != first[1]))
+    kv.close()
+    assert np.mean(differ) < 5e-3, np.mean(differ)
