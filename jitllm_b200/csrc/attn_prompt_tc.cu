@@ -19,6 +19,8 @@
 // What bounds it: 4.3 us per 128 keys against 0.8 us of tensor work and about 1.1 us of exponentials. Without copies after
 // the second tile the 8192-token prompt was 7 % faster, without the exponentials 16 %: the softmax warps' chain (two passes
 // over the scores, two row barriers, adding the tile's O) comes first, then the copies.
+// The tensor-memory instructions and the row barriers are .sync.aligned: each follows a __syncwarp() or a vote behind whatever
+// may have split the warp (a lane's arrival, a poll that lanes leave at different times).
 // Roles: warps 0-7 softmax and output, warps 8-9 copy keys, 10-11 values (cp.async, a ring of two tiles each), warp 12
 // issues the MMAs. They meet at mbarriers; every wait is bounded and a wait that runs out sets the status word.
 #include "gemm_tc_core.cuh"
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
             constexpr uint32_t idesc_s = (1u << 4) | (uint32_t(kPtKeys >> 3) << 17) | (uint32_t(kPtRows >> 4) << 24);
             constexpr uint32_t idesc_o = (1u << 4) | (1u << 16) | (uint32_t(HD >> 3) << 17) | (uint32_t(kPtRows >> 4) << 24);
             const uint32_t q0 = smem_u32(base + S::q_off), k0 = smem_u32(base + S::k_off), v0 = smem_u32(base + S::v_off);
-            ok = mbar_poll_bounded(q_full, 0);
+            ok = __all_sync(0xffffffffu, mbar_poll_bounded(q_full, 0));
             for (int t = 0; t <= tiles && ok && *abort_flag == 0u; ++t) {
                 const int b = t & 1;
                 if (t < tiles) {
@@ -304,12 +306,16 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
         const float scale = 1.4426950408889634f / sqrtf(static_cast<float>(HD));
         const uint32_t lanes = uint32_t((warp & 3) * 32) << 16;
         // the two warps that share these 32 rows
-        const auto row_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory"); };
+        const auto row_sync = [&]() {
+            __syncwarp();
+            asm volatile("bar.sync %0, 64;" ::"r"(1 + (warp & 3)) : "memory");
+        };
         // A wait that ran out is noted, and the loop goes on to its end so that the two warps of a row stay in step; later
         // waits poll once, and nothing it computes is used (the status word is set).
         bool all_ok = true;
         const auto add_o = [&](int t) {  // o = o * corr + the O of tile t
             ok = mbar_spin_bounded(o_full, uint32_t(t) & 1u, all_ok ? (1u << 26) : 1u);
+            __syncwarp();
             tc_fence_after();
 #pragma unroll
             for (int g = 0; g < kDims / 16; ++g) {
@@ -322,6 +328,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
         for (int t = 0; t < tiles; ++t) {
             ok = mbar_spin_bounded(s_full + (t & 1), uint32_t(t >> 1) & 1u, all_ok ? (1u << 26) : 1u);
             all_ok = all_ok && ok;
+            __syncwarp();
             tc_fence_after();
             // The scores are read twice, for the maximum and for the exponentials: with the 64 sums they do not fit the
             // registers at once (128 a thread: one scheduler holds four of the thirteen warps).
@@ -379,6 +386,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
             if (t > 0) add_o(t - 1);
             all_ok = all_ok && ok;
             corr = next_corr;
+            __syncwarp();
             {
                 uint32_t c[16];
 #pragma unroll

@@ -151,11 +151,16 @@ struct TileOut {
     bool inside;       // the row exists
 };
 
+// The tensor-memory instructions below are .sync.aligned: the whole warp executes each of them together. Whatever may have
+// split it (a lane's arrival, a poll that lanes leave at different times, a row past the matrix) is followed by a
+// __syncwarp() or a vote before the next one.
+
 // This CTA's partial tile into its slot: 16-column groups g0, g0 + step, ... of the accumulator.
 __device__ __forceinline__ void store_partial(const TileOut &o, uint32_t acc, int g0, int step) {
 #pragma unroll 1
     for (int c0 = g0 * 16; c0 < o.ntok; c0 += step * 16) {
         float v[16];
+        __syncwarp();
         tmem_ld16(acc + uint32_t(c0), v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) o.slot[size_t(c0 + j) * kTileM] = v[j];
@@ -179,6 +184,7 @@ __device__ __forceinline__ void finish_tile(const GemmArgs &a, const TileOut &o,
 #pragma unroll 1
         for (int c = c_first; c <= c_last; ++c) {
             if (c == own) {
+                __syncwarp();
                 tmem_ld16(acc + uint32_t(c0), v);
             } else {
                 // only the first contributor's range starts before the tile
@@ -189,14 +195,15 @@ __device__ __forceinline__ void finish_tile(const GemmArgs &a, const TileOut &o,
 #pragma unroll
             for (int j = 0; j < 16; ++j) sum[j] = c == c_first ? v[j] : sum[j] + v[j];
         }
-        if (!o.inside) continue;
-        if (o.res != nullptr) {
+        if (o.inside) {
+            if (o.res != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) sum[j] = res[j] + sum[j];
+                for (int j = 0; j < 16; ++j) sum[j] = res[j] + sum[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (c0 + j < o.ntok) o.y[size_t(c0 + j) * o.rows] = sum[j];
         }
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-            if (c0 + j < o.ntok) o.y[size_t(c0 + j) * o.rows] = sum[j];
     }
 }
 
@@ -367,7 +374,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 const int u_hi = (f / raw_total + 1) * raw_total;
                 const int seg_end = u_hi < hi ? u_hi : hi;
                 const int nstage = 8 * (seg_end - f);
-                if (turn > 0) ok = wait_pair(smem_u32(acc_empty), uint32_t(turn - 1) & 1u);
+                if (turn > 0) ok = __all_sync(0xffffffffu, wait_pair(smem_u32(acc_empty), uint32_t(turn - 1) & 1u));
                 for (int k = 0; k < nstage && ok; ++k) {
                     ok = wait_pair(a_full0 + 8u * uint32_t(sa), pa) && wait_pair(b_full0 + 8u * uint32_t(sb), pb);
                     if (!__all_sync(0xffffffffu, ok)) {
@@ -411,6 +418,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             tc_fence_before();
             __syncwarp();
             if (lane == 0) arrive_cluster(a_full_lead + 8u * uint32_t(pending));
+            __syncwarp();
             pending = -1;
         };
         int s = grp, rev = 0, st = 0, unit = grp;
@@ -453,7 +461,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         }
         if (ok) publish();
         // The range's last tile, if this pair finishes it: these warps are idle by then.
-        if (ok) ok = mbar_poll_bounded(last_fold, 0u);
+        if (ok) ok = __all_sync(0xffffffffu, mbar_poll_bounded(last_fold, 0u));
         if (ok && last_flags[0] != 0u) {
             const int u = (hi - 1) / raw_total;
             tc_fence_after();
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             if (lane == 0) mbar_arrive(epi_bar);
             const bool there = mbar_poll_bounded(epi_bar, uint32_t(epi_phase) & 1u);
             ++epi_phase;
-            return there;
+            return bool(__all_sync(0xffffffffu, there));
         };
         int f = lo;
         while (f < hi && *abort_flag == 0u) {

@@ -35,7 +35,7 @@ def _tensor_memory_kernels():
                 yield pytest.param(body, id=f"{path.name}:{name}")
 
 
-@pytest.mark.parametrize("body", _tensor_memory_kernels())
+@pytest.mark.parametrize("body", list(_tensor_memory_kernels()))
 def test_dependents_are_released_after_the_tensor_memory_is_allocated(body):
     """A dependent kernel's CTA that lands on the SM of a CTA which has not allocated yet could take the tensor memory and
     then wait for that CTA's grid to finish: neither would ever go on."""
@@ -43,3 +43,22 @@ def test_dependents_are_released_after_the_tensor_memory_is_allocated(body):
     barrier = body.index("__syncthreads()", alloc)  # the allocating warp has passed it with its columns
     release = [m.start() for m in re.finditer(r"pdl_launch_dependents\(\)", body)]
     assert release and min(release) > barrier
+
+
+ALIGNED = re.compile(r"tmem_ld16\(|tmem_st16\(|tmem_wait_st\(\)|bar\.sync ")
+SPLITS = re.compile(r"lane == 0|tid == 0|mbar_poll_bounded\w*\(|mbar_spin_bounded\(|wait_pair\(|\.inside|\bcontinue;")
+JOINS = re.compile(r"__syncwarp\(\)|__all_sync\([^;]*;|__any_sync\([^;]*;|__syncthreads\(\)|cluster_sync_all\(\)")
+
+
+@pytest.mark.parametrize("name", ["gemm_wide.cu", "attn_prompt_tc.cu"])
+def test_warps_are_whole_where_aligned_instructions_stand(name):
+    """tcgen05.ld / st / wait and bar.sync are .sync.aligned: executed by a warp that is split, they are undefined. Between
+    anything that can split it and the next such instruction stands something that joins it again, in the order of the text."""
+    text = _code(CSRC / name)
+    places = [m.start() for m in ALIGNED.finditer(text)]
+    assert places
+    joins = [m.end() for m in JOINS.finditer(text)]
+    splits = [m.start() for m in SPLITS.finditer(text)]
+    for at in places:
+        split = max((s for s in splits if s < at), default=-1)
+        assert split < 0 or any(split < j <= at for j in joins), text[:at].count("\n") + 1
