@@ -1135,10 +1135,23 @@ int run_step(jl_ctx *ctx, int width, bool with_logits, bool advance = false) {
     return JL_OK;
 }
 
+// After a wait that ran out: the status word, and every arrival counter. Kernels find those at zero and leave them so, but
+// one that gave up may have counted part of its arrivals; the next one would take them for its own and finish a tile from
+// partial results that are not there yet.
+cudaError_t clear_after_timeout(jl_ctx *ctx) {
+    cudaError_t e = cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->gemm_counters, 0, kGemmCounters * sizeof(unsigned), ctx->stream);
+    if (e == cudaSuccess && ctx->att_count)
+        e = cudaMemsetAsync(ctx->att_count, 0, size_t(ctx->row_cap) * ctx->l_kv_heads * sizeof(unsigned), ctx->stream);
+    if (e == cudaSuccess && ctx->amax_count)
+        e = cudaMemsetAsync(ctx->amax_count, 0, size_t(ctx->desc.max_batch) * sizeof(unsigned), ctx->stream);
+    return e;
+}
+
 int check_status(jl_ctx *ctx) {
     int st = ctx->h_stage[5 * ctx->row_cap];
     if (st == kDevTimeout) {
-        cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+        JL_CUDA(ctx, clear_after_timeout(ctx));
         return fail(ctx, JL_ERR_TIMEOUT, "a kernel gave up waiting for an asynchronous copy");
     }
     return JL_OK;
@@ -2180,7 +2193,7 @@ int32_t jl_gemv(jl_ctx *ctx, int32_t ggml_type, int64_t rows, int64_t cols, cons
     if (rc) return rc;
     if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "matrix-vector product failed: %s", cudaGetErrorString(e));
     if (status == kDevTimeout) {
-        cudaMemset(ctx->d_status, 0, 4);
+        JL_CUDA(ctx, clear_after_timeout(ctx));
         return fail(ctx, JL_ERR_TIMEOUT, "a kernel gave up waiting for an asynchronous copy");
     }
     ctx->counters.h2d_bytes += size_t(n) * cols * 4;
@@ -2308,7 +2321,7 @@ int32_t jl_debug_peer_wait_timeout(jl_ctx *ctx, int32_t timeout_ms) {
     int status = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&status, ctx->d_status, sizeof status, cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
+    if (e == cudaSuccess && status == kDevTimeout) e = clear_after_timeout(ctx);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(buf);
     if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "peer wait self-test failed: %s", cudaGetErrorString(e));

@@ -62,3 +62,16 @@ def test_warps_are_whole_where_aligned_instructions_stand(name):
     for at in places:
         split = max((s for s in splits if s < at), default=-1)
         assert split < 0 or any(split < j <= at for j in joins), text[:at].count("\n") + 1
+
+
+def test_a_timeout_clears_every_arrival_counter_with_the_status_word():
+    """A launch that gave up leaves its counters partly counted. The status word is therefore reset (but for its
+    allocation) in one function only, and that function zeroes each device counter the context holds."""
+    text = _code(CSRC / "engine.cu")
+    clear = _function_at(text, text.index("cudaError_t clear_after_timeout("))
+    resets = re.findall(r"cudaMemset(?:Async)?\(ctx->d_status", text)
+    assert len(resets) == len(re.findall(r"cudaMemset(?:Async)?\(ctx->d_status", clear)) + 1  # jl_init
+    counters = set(re.findall(r"unsigned \*(\w*count\w*) = nullptr", text))
+    assert counters == {"gemm_counters", "att_count", "amax_count"}
+    for name in counters:
+        assert f"cudaMemsetAsync(ctx->{name}, 0," in clear, name
