@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
             constexpr uint32_t idesc_s = (1u << 4) | (uint32_t(kPtKeys >> 3) << 17) | (uint32_t(kPtRows >> 4) << 24);
             constexpr uint32_t idesc_o = (1u << 4) | (1u << 16) | (uint32_t(HD >> 3) << 17) | (uint32_t(kPtRows >> 4) << 24);
             const uint32_t q0 = smem_u32(base + S::q_off), k0 = smem_u32(base + S::k_off), v0 = smem_u32(base + S::v_off);
+            int keys_in = 0, values_in = 0;  // tiles whose MMAs have been issued
             ok = __all_sync(0xffffffffu, mbar_poll_bounded(q_full, 0));
             for (int t = 0; t <= tiles && ok && *abort_flag == 0u; ++t) {
                 const int b = t & 1;
@@ -176,6 +177,7 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
                     }
                     umma_commit_one(s_full + b);
                     umma_commit_one(k_empty + b);
+                    ++keys_in;
                 }
                 if (t > 0) {
                     const int pb = (t - 1) & 1;
@@ -192,12 +194,12 @@ __global__ void __launch_bounds__(kPtThreads, 1) attn_prompt_tc_kernel(const Att
                                 pt_desc(v0 + uint32_t(pb) * S::tile + uint32_t(k) * 2048u, S::atom), idesc_o, k > 0 ? 1u : 0u);
                     umma_commit_one(o_full);
                     umma_commit_one(v_empty + pb);
+                    ++values_in;
                 }
             }
-            // the last hand-backs have arrived before this CTA leaves
-            for (int t = tiles > 2 ? tiles - 2 : 0; t < tiles && ok; ++t)
-                ok = mbar_poll_bounded(k_empty + (t & 1), uint32_t(t >> 1) & 1u) &&
-                     mbar_poll_bounded(v_empty + (t & 1), uint32_t(t >> 1) & 1u);
+            // The MMAs are over and the last hand-backs have arrived before this CTA leaves, whatever ended the loop.
+            for (int t = max(keys_in - 2, 0); t < keys_in; ++t) ok = mbar_poll_bounded(k_empty + (t & 1), uint32_t(t >> 1) & 1u) && ok;
+            for (int t = max(values_in - 2, 0); t < values_in; ++t) ok = mbar_poll_bounded(v_empty + (t & 1), uint32_t(t >> 1) & 1u) && ok;
         }
     } else if (warp >= kPtSoftWarps) {
         // ---- key and value tiles, past the last key zeros -------------------------------------------------

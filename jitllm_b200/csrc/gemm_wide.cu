@@ -99,6 +99,12 @@ __device__ __forceinline__ bool wait_pair(uint32_t bar, uint32_t parity, uint32_
     }
     return false;
 }
+// A word at the same place in the shared memory of either CTA of the pair (rank 0 or 1).
+__device__ __forceinline__ void store_in_cta(uint32_t smem_addr, uint32_t rank, uint32_t value) {
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.u32 [a], %2;\n\t}" ::"r"(smem_addr),
+                 "r"(rank), "r"(value)
+                 : "memory");
+}
 // One activation box into this CTA's shared memory, completing on a barrier of the pair's first CTA.
 __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap *map, int x, int y, uint32_t leader_bar) {
     asm volatile(
@@ -140,6 +146,29 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
         "mov.b16 mask, 3;\n\t"
         "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], mask;\n\t}"
         ::"r"(bar) : "memory");
+}
+
+// The last of the stages 0 .. issued - 1 that went through slot s of a ring, or -1.
+constexpr __host__ __device__ int last_in_slot(int issued, int s, int slots) {
+    return issued > s ? issued - 1 - (issued - 1 - s) % slots : -1;
+}
+static_assert(last_in_slot(0, 0, 8) == -1 && last_in_slot(5, 5, 8) == -1 && last_in_slot(6, 5, 8) == 5, "first round");
+static_assert(last_in_slot(8, 7, 8) == 7 && last_in_slot(9, 0, 8) == 8 && last_in_slot(9, 1, 8) == 1, "second round");
+
+// Waits in the pair's first CTA for the activation boxes of both that a launch which gave up has left on their way: issued0
+// and issued1 of the CTAs' stages. They complete on this CTA's barriers, a phase per stage, so the latest phase of a slot is
+// armed for what will still arrive there: both boxes, or the one CTA's if the other has stopped a round earlier.
+__device__ __forceinline__ void drain_activations(uint64_t *b_full, int slots, uint32_t stage_bytes, int issued0, int issued1) {
+    for (int s = 0; s < slots; ++s) {
+        const int last0 = last_in_slot(issued0, s, slots), last1 = last_in_slot(issued1, s, slots);
+        const int last = last0 > last1 ? last0 : last1;
+        if (last < 0) continue;
+        if (last0 < last) mbar_expect_tx(b_full + s, stage_bytes);
+        if (last1 < last)
+            asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b_full + s)), "r"(stage_bytes)
+                         : "memory");
+        mbar_poll_bounded(b_full + s, uint32_t(last / slots) & 1u);
+    }
 }
 
 // Where a pair's share of a tile goes and what is added to it on the way.
@@ -230,11 +259,13 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     uint64_t *epi_bar = acc_empty + 1;     // the epilogue warps' own barrier
     uint64_t *last_fold = epi_bar + 1;     // it is known whether the range's last tile is finished here
     static_assert(BS <= AS, "activation stages");
-    static_assert((2 * AS + BS + 2 * 4 + 4) * 8 + 80 <= S::bar_bytes, "barrier block");
+    static_assert((2 * AS + BS + 2 * 4 + 4) * 8 + 96 <= S::bar_bytes, "barrier block");
     uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(base + S::bar_off + S::bar_bytes - 16);
     volatile uint32_t *fold_flags = reinterpret_cast<uint32_t *>(base + S::bar_off + S::bar_bytes - 64);  // four, taken in turn
     volatile uint32_t *last_flags = fold_flags - 4;
     volatile uint32_t *abort_flag = tmem_ptr + 2;
+    // The same in both CTAs at the end: the activation stages that either has issued, and whether either gave up.
+    volatile uint32_t *pair_issued = last_flags - 4, *pair_abort = pair_issued + 2;
 
     int tiles = 0;
     for (int s = 0; s < a.nseg; ++s) tiles += (a.seg[s].rows + kPairM - 1) / kPairM;
@@ -266,6 +297,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
         mbar_init(last_fold, 1);
         mbar_fence_init();
         *abort_flag = 0u;
+        pair_abort[0] = pair_abort[1] = 0u;
     }
     tc_fence_before();
     __syncthreads();
@@ -329,8 +361,8 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                                           raw_full + st);
                 }
             }
-            if (!ok || *abort_flag != 0u)  // winding down: no copy may still be on its way into this CTA
-                for (int k = i > RS ? i - RS : 0; k < i; ++k) mbar_poll_bounded(raw_full + k % RS, uint32_t(k / RS) & 1u);
+            // no copy may still be on its way into this CTA (after a wait that ran out: nobody may have read them)
+            for (int k = i > RS ? i - RS : 0; k < i; ++k) mbar_poll_bounded(raw_full + k % RS, uint32_t(k / RS) & 1u);
         }
     } else if (warp == kEpiWarps + kConvWarps + 2) {
         // ---- activation rows: this CTA's 128 tokens of the tile, the lo parts, then the hi parts ------------
@@ -351,13 +383,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                                      (k < len ? a.x_lo_row : 0) + tok, leader_addr(smem_u32(b_full + s)));
                 }
             }
-            if (!ok || *abort_flag != 0u) {
-                if (rank == 0)
-                    for (int k = q > BS ? q - BS : 0; k < q; ++k) mbar_poll_bounded(b_full + k % BS, uint32_t(k / BS) & 1u);
-            } else {  // every hand-back has arrived here before this CTA may leave
+            for (uint32_t r = 0; r < 2; ++r) store_in_cta(smem_u32(const_cast<uint32_t *>(pair_issued + rank)), r, uint32_t(q));
+            // every hand-back has arrived here before this CTA may leave
+            if (*abort_flag == 0u)
                 for (int k = stages > AS ? stages - AS : 0; k < stages && ok; ++k)
                     ok = mbar_poll_bounded(done + k % AS, uint32_t(k / AS) & 1u);
-            }
         }
     } else if (warp == kEpiWarps + kConvWarps) {
         // ---- tensor-core issue (first CTA of the pair) -----------------------------------------------------
@@ -367,7 +397,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
             constexpr uint32_t desc_hi = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);  // SBO, version, 128-byte swizzle
             const uint32_t b_lo0 = ((smem_u32(base) >> 4) & 0x3FFFu) | (1u << 16);
             const uint32_t a_full0 = smem_u32(a_full), done0 = smem_u32(done), b_full0 = smem_u32(b_full);
-            int sa = 0, sb = 0, turn = 0;
+            int sa = 0, sb = 0, turn = 0, issued = 0;
             uint32_t pa = 0, pb = 0;
             int f = lo;
             while (f < hi && ok && *abort_flag == 0u) {
@@ -385,6 +415,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                     umma_stage_pair(tmem_d, tmem_d + kAccCols + uint32_t(sa) * kAStageCols,
                                     b_lo0 + uint32_t(sb) * uint32_t(S::b_stage >> 4), desc_hi, idesc, done0 + 8u * uint32_t(sa),
                                     k == 0 ? 0u : 1u);
+                    ++issued;
                     if (++sa == AS) {
                         sa = 0;
                         pa ^= 1u;
@@ -402,6 +433,9 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 ++turn;
                 f = seg_end;
             }
+            // the MMAs are over before the tensor memory is given back, whatever ended the loop
+            if (issued > 0) wait_pair(done0 + 8u * uint32_t((issued - 1) % AS), uint32_t((issued - 1) / AS) & 1u);
+            __syncwarp();
         }
     } else if (warp >= kEpiWarps) {
         // ---- conversion: groups of four warps take the units in turn --------------------------------------
@@ -459,7 +493,11 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                 }
             }
         }
-        if (ok) publish();
+        __syncwarp();
+        if (ok)
+            publish();
+        else
+            tmem_wait_st();  // no store may be on its way when the tensor memory is given back
         // The range's last tile, if this pair finishes it: these warps are idle by then.
         if (ok) ok = __all_sync(0xffffffffu, mbar_poll_bounded(last_fold, 0u));
         if (ok && last_flags[0] != 0u) {
@@ -560,7 +598,15 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     __syncwarp();
     tc_fence_before();
     __syncthreads();
+    if (tid == 0 && *abort_flag != 0u)
+        for (uint32_t r = 0; r < 2; ++r) store_in_cta(smem_u32(const_cast<uint32_t *>(pair_abort + rank)), r, 1u);
+    __syncwarp();
     cluster_sync_all();  // neither CTA leaves while the other may still reach into it
+    if ((pair_abort[0] | pair_abort[1]) != 0u) {
+        if (rank == 0 && tid == 0) drain_activations(b_full, BS, S::b_stage, int(pair_issued[0]), int(pair_issued[1]));
+        __syncwarp();
+        cluster_sync_all();
+    }
     if (warp == kEpiWarps + kConvWarps)
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kWideTmemCols) : "memory");
 }

@@ -75,3 +75,20 @@ def test_a_timeout_clears_every_arrival_counter_with_the_status_word():
     assert counters == {"gemm_counters", "att_count", "amax_count"}
     for name in counters:
         assert f"cudaMemsetAsync(ctx->{name}, 0," in clear, name
+
+
+def test_what_is_on_its_way_is_waited_for_whatever_ended_the_kernel():
+    """A launch that gave up leaves in order too: copies into a CTA's shared memory and MMAs on its tensor memory are over
+    before the CTA is. The pair's first CTA, on whose barriers the activation boxes of both complete, waits for them behind
+    the barrier that both pass when nothing more is issued, and the second stays until it has; the issuing warps wait for
+    their last commits without looking at how the loop ended."""
+    wide = _code(CSRC / "gemm_wide.cu")
+    kernel = _function_at(wide, wide.index("__global__"))
+    drain = kernel.index("drain_activations(")
+    assert kernel.rindex("cluster_sync_all()", 0, drain) and kernel.index("cluster_sync_all()", drain) < kernel.index("tcgen05.dealloc")
+    assert "if (issued > 0) wait_pair(done0" in kernel
+    assert re.search(r"\n            for \(int k = i > RS \? i - RS : 0; k < i; \+\+k\) mbar_poll_bounded\(raw_full", kernel)
+    attention = _code(CSRC / "attn_prompt_tc.cu")
+    for done in ("k_empty", "v_empty"):
+        loop = re.search(r"for \(int t = max\(\w+ - 2, 0\); ([^;]*); \+\+t\) ok = mbar_poll_bounded\(" + done, attention)
+        assert loop and "ok" not in loop.group(1), done
