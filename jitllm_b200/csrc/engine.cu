@@ -112,7 +112,8 @@ struct jl_ctx {
     float *gemm_scratch = nullptr;       // split-column partial tiles of the tensor-core path
     size_t gemm_scratch_floats = 0;
     unsigned *gemm_counters = nullptr;   // one arrival counter per output tile, zero between launches
-    void *split_ws = nullptr;            // stand-alone products: one slab of activation rows as binary16 hi / lo parts
+    void *split_ws = nullptr;            // stand-alone products of more than 64 rows (from the first on): a slab of
+                                         // activation rows as binary16 hi / lo parts
     float *part = nullptr;      // row-parallel partial sums before the all-reduce, [row_cap][dim]
     float *best = nullptr;      // local (value, index) of the arg-max and the gathered pairs
     // peer-memory exchange (tp_exchange.cuh): this GPU's inbox, every rank's inbox as mapped here
@@ -773,15 +774,32 @@ int launch_gemm_segs(jl_ctx *ctx, const DevTensor *const *w, float *const *y, co
     return JL_OK;
 }
 
+// The workspace of launch_product, held from the first product that wants it to the end of the context. False if it cannot
+// be had now: no memory left for it, or the stream is being captured (another stream's capture is left alone).
+bool split_workspace(jl_ctx *ctx) {
+    if (ctx->split_ws) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) return false;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaMalloc(&ctx->split_ws, kSplitWsBytes) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->split_ws = nullptr;
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return ctx->split_ws != nullptr;
+}
+
 // A stand-alone product. More rows than one token tile of the in-kernel conversion (64) have their activations split
 // into binary16 parts first, by slabs that fit the workspace: converting them inside the product kernel repeats that
-// work for every 128 weight rows.
+// work for every 128 weight rows. It is what remains without a workspace, and for rows too long for 256 of them to fit it
+// (more than 65536 columns).
 int launch_product(jl_ctx *ctx, const DevTensor &w, const float *x, int n, float *y, uint64_t *launches) {
     const size_t cols = size_t(w.cols);
     size_t slab = kSplitWsBytes / (4 * cols) / 256 * 256;
     const size_t row_tiles = (size_t(w.rows) + 255) / 256;  // two arrival counters per 256 x 256 output tile
     if (slab > kGemmCounters / 2 / row_tiles * 256) slab = kGemmCounters / 2 / row_tiles * 256;
-    if (n <= 64 || slab < 256) return launch_gemm(ctx, w, x, n, y, nullptr, launches);
+    if (n <= 64 || slab < 256 || !split_workspace(ctx)) return launch_gemm(ctx, w, x, n, y, nullptr, launches);
     for (size_t t0 = 0; t0 < size_t(n); t0 += slab) {
         const int rows = int(std::min(slab, size_t(n) - t0));
         char *hi = static_cast<char *>(ctx->split_ws), *lo = hi + size_t(rows) * cols * 2;
@@ -1207,7 +1225,6 @@ int32_t jl_init(int32_t device_id, jl_ctx **out) {
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->gemm_scratch), kGemmScratchFloats * 4);
     if (e == cudaSuccess) ctx->gemm_scratch_floats = kGemmScratchFloats;
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->split_ws, kSplitWsBytes);
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void **>(&ctx->gemm_counters), kGemmCounters * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(ctx->gemm_counters, 0, kGemmCounters * sizeof(unsigned));
     if (e != cudaSuccess) {

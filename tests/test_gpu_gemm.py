@@ -133,3 +133,55 @@ def test_wide_product_is_as_close_to_64_bits_as_the_narrow_one(dev):
         err[m] = np.linalg.norm(got[:128] - want[:128]) / np.linalg.norm(want[:128])
     assert err[n] < 256 * 2.0 ** -24, err
     assert err[n] <= 1.05 * err[128], err
+
+
+def test_split_workspace_is_there_from_the_first_wide_product_on(built):
+    """A context that never multiplies a stand-alone matrix by more than 64 rows does not hold the 64 MiB their activations
+    are split into; the first that does takes it, later ones find it, and it goes with the context."""
+    import torch
+    t, rows, cols = GGMLType.Q8_0, 256, 512
+    w = jl.synth_tensor(t, rows * cols, seed=3)
+    x = np.random.default_rng(3).standard_normal((70, cols)).astype(np.float32)
+    free = lambda: torch.cuda.mem_get_info(0)[0] / 2 ** 20
+    with jl.Device(0) as warm:  # the kernels' code is loaded once per process
+        want = warm.matmul(t, w, rows, cols, x)
+        warm.matmul(t, w, rows, cols, x[:64])
+        before = free()
+        with jl.Device(0) as d:
+            narrow = d.matmul(t, w, rows, cols, x[:64])
+            held = before - free()
+            assert held < 64 + 32, held  # the products' own scratch is 64 MiB
+            assert np.array_equal(d.matmul(t, w, rows, cols, x), want)
+            assert 60 <= before - free() - held <= 70
+            assert np.array_equal(d.matmul(t, w, rows, cols, x), want)
+            assert 60 <= before - free() - held <= 70
+        assert abs(before - free()) < 8
+    assert np.linalg.norm(narrow - want[:64]) < EXPECT * np.linalg.norm(want[:64])
+
+
+@pytest.mark.parametrize("rows,cols,n", [(300, 512, 100),        # two token tiles of the in-kernel conversion
+                                         (128256, 256, 1100)])   # and more tiles than arrival counters: two token slabs
+def test_wide_product_inside_a_capture(built, oracle, rows, cols, n):
+    """The first wide product of a context while its stream is being captured, where no memory can be taken: the activations
+    are converted inside the product kernel, the capture stays whole, and its replay gives the product."""
+    import torch
+    t = GGMLType.Q4_0
+    w = jl.synth_tensor(t, rows * cols, seed=23)
+    x = np.random.default_rng(7).standard_normal((n, cols)).astype(np.float32)
+    with jl.Device(0) as d:
+        m = d.upload_matrix(t, w, rows, cols)
+        xd, yd = d.alloc(x.nbytes), d.alloc(n * rows * 4)
+        d.h2d(xd, x)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(d._lib.jl_stream(d.handle))):
+            m.matmul_dev(xd, n, yd)
+        graph.replay()
+        torch.cuda.synchronize()
+        got = np.empty((n, rows), np.float32)
+        d.d2h(got, yd)
+        del graph
+        m.close()
+    sample = sorted({0, 63, 64, 65, n // 2, n - 1} | ({1023, 1024, 1025} & set(range(n))))
+    want = oracle.matmul(t, w, x[sample], rows, cols)
+    err = np.linalg.norm(got[sample] - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() < EXPECT, err
