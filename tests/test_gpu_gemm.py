@@ -61,9 +61,10 @@ def test_wide_activations_do_not_overflow_fp16(dev, oracle):
     assert rel_l2(got, want) < EXPECT
 
 
-def test_tall_product_goes_in_token_slabs(dev, oracle):
-    """More output tiles than arrival counters (1002 row tiles x 18 token tiles): the launch is cut into
-    token slabs; sampled rows against the oracle and two slabs' boundary rows included."""
+def test_tall_product(dev, oracle):
+    """The most weight rows against more than a thousand activation rows: 501 row tiles by five token tiles in one launch, an
+    arrival counter for either CTA of each. (Without the workspace of the split activations the same product goes in token
+    slabs: test_wide_product_inside_a_capture.)"""
     rows, cols, n, t = 128256, 256, 1100, GGMLType.Q4_0
     w = jl.synth_tensor(t, rows * cols, seed=23)
     x = np.random.default_rng(7).standard_normal((n, cols)).astype(np.float32)
@@ -133,6 +134,22 @@ def test_wide_product_is_as_close_to_64_bits_as_the_narrow_one(dev):
         err[m] = np.linalg.norm(got[:128] - want[:128]) / np.linalg.norm(want[:128])
     assert err[n] < 256 * 2.0 ** -24, err
     assert err[n] <= 1.05 * err[128], err
+
+
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q8_0])
+@pytest.mark.parametrize("tail", [9, 33, 100, 300])  # a second slab for the 16-, 64- and 128-row kernels and the CTA pairs
+def test_wide_product_in_two_slabs(dev, oracle, t, tail):
+    """14336 columns: 1024 rows of split activations fill the workspace, the rest go in a second slab with a descriptor of
+    its own, behind the first slab's product on the same buffer."""
+    rows, cols, n = 300, 14336, 1024 + tail
+    w = jl.synth_tensor(t, rows * cols, seed=tail)
+    x = np.random.default_rng(tail).standard_normal((n, cols)).astype(np.float32)
+    got = dev.matmul(t, w, rows, cols, x)
+    sample = [0, 255, 256, 1022, 1023, 1024, 1025, n - 2, n - 1]
+    want = oracle.matmul(t, w, x[sample], rows, cols)
+    err = np.linalg.norm(got[sample] - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() < EXPECT, err
+    assert np.all(np.isfinite(got))
 
 
 def test_split_workspace_is_there_from_the_first_wide_product_on(built):
