@@ -4,9 +4,10 @@
 
 #include <dlfcn.h>
 
+#include <algorithm>
+#include <iterator>
 #include <set>
 
-#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -107,7 +108,7 @@ struct jl_ctx {
     // descriptors per token-tile size (16, 32, 64): [0] xb as rows of dim, [1] xb as rows of the
     // local query width, [2] hb as rows of the local hidden width
     void *xb16 = nullptr, *hb16 = nullptr;
-    GemmTensorMap xmaps[3][4] = {};
+    GemmTensorMap xmaps[3][std::size(kGemmBoxes)] = {};
     GemmTensorMap wcls_slice_tmap = {};  // tied embeddings under tensor parallelism: this GPU's rows
     float *gemm_scratch = nullptr;       // split-column partial tiles of the tensor-core path
     size_t gemm_scratch_floats = 0;
@@ -758,8 +759,8 @@ int launch_gemm_segs(jl_ctx *ctx, const DevTensor *const *w, float *const *y, co
             if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "activation split launch failed: %s", cudaGetErrorString(e));
             ++*launches;
         }
-        const int nt = gemm_token_tile(n);
-        g.xmap = &ctx->xmaps[in_kind][nt == 16 ? 0 : (nt == 32 ? 1 : (nt == 64 ? 2 : 3))];
+        const int *box = std::find(std::begin(kGemmBoxes), std::end(kGemmBoxes), gemm_box_rows(n));
+        g.xmap = &ctx->xmaps[in_kind][box - std::begin(kGemmBoxes)];
         g.x_lo_row = ctx->row_cap;
     }
     g.nseg = nseg;
@@ -792,14 +793,14 @@ bool split_workspace(jl_ctx *ctx) {
 
 // A stand-alone product. More rows than one token tile of the in-kernel conversion (64) have their activations split
 // into binary16 parts first, by slabs that fit the workspace: converting them inside the product kernel repeats that
-// work for every 128 weight rows. It is what remains without a workspace, and for rows too long for 256 of them to fit it
-// (more than 65536 columns).
+// work for every 128 weight rows. It is what remains without a workspace, and for rows too long for 192 of them to fit it
+// (more than 87381 columns).
 int launch_product(jl_ctx *ctx, const DevTensor &w, const float *x, int n, float *y, uint64_t *launches) {
     const size_t cols = size_t(w.cols);
-    size_t slab = kSplitWsBytes / (4 * cols) / 256 * 256;
-    const size_t row_tiles = (size_t(w.rows) + 255) / 256;  // two arrival counters per 256 x 256 output tile
-    if (slab > kGemmCounters / 2 / row_tiles * 256) slab = kGemmCounters / 2 / row_tiles * 256;
-    if (n <= 64 || slab < 256 || !split_workspace(ctx)) return launch_gemm(ctx, w, x, n, y, nullptr, launches);
+    size_t slab = kSplitWsBytes / (4 * cols) / 192 * 192;   // whole tiles of the CTA-pair kernel
+    const size_t row_tiles = (size_t(w.rows) + 255) / 256;  // two arrival counters per output tile
+    if (slab > kGemmCounters / 2 / row_tiles * 192) slab = kGemmCounters / 2 / row_tiles * 192;
+    if (n <= 64 || slab < 192 || !split_workspace(ctx)) return launch_gemm(ctx, w, x, n, y, nullptr, launches);
     for (size_t t0 = 0; t0 < size_t(n); t0 += slab) {
         const int rows = int(std::min(slab, size_t(n) - t0));
         char *hi = static_cast<char *>(ctx->split_ws), *lo = hi + size_t(rows) * cols * 2;
@@ -807,7 +808,7 @@ int launch_product(jl_ctx *ctx, const DevTensor &w, const float *x, int n, float
         if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "activation split launch failed: %s", cudaGetErrorString(e));
         ++*launches;
         GemmTensorMap xmap;
-        e = gemm_make_activation_map(&xmap, hi, rows, int64_t(cols), gemm_token_tile(rows));
+        e = gemm_make_activation_map(&xmap, hi, rows, int64_t(cols), gemm_box_rows(rows));
         if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "activation descriptor failed: %s", cudaGetErrorString(e));
         GemmArgs g = gemm_args(ctx, w, rows);
         g.seg[0] = {w.data, &w.tmap, y + t0 * size_t(w.rows), nullptr, int(w.rows)};
@@ -1504,11 +1505,10 @@ int32_t jl_model_finalize(jl_ctx *ctx) {
     {
         if ((rc = alloc(&ctx->xb16, 2 * R * d.dim * 2))) return rc;
         if ((rc = alloc(&ctx->hb16, 2 * R * ctx->l_hidden * 2))) return rc;
-        const int nts[4] = {16, 32, 64, 128};
-        for (int i = 0; i < 4; ++i) {
-            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[0][i], ctx->xb16, R, d.dim, nts[i]));
-            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[1][i], ctx->xb16, R, ctx->l_qdim, nts[i]));
-            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[2][i], ctx->hb16, R, ctx->l_hidden, nts[i]));
+        for (size_t i = 0; i < std::size(kGemmBoxes); ++i) {
+            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[0][i], ctx->xb16, R, d.dim, kGemmBoxes[i]));
+            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[1][i], ctx->xb16, R, ctx->l_qdim, kGemmBoxes[i]));
+            JL_CUDA(ctx, gemm_make_activation_map(&ctx->xmaps[2][i], ctx->hb16, R, ctx->l_hidden, kGemmBoxes[i]));
         }
     }
     if (ctx->tp_size > 1) {

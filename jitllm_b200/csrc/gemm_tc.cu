@@ -853,10 +853,13 @@ cudaError_t gemm_make_tensor_map(GemmTensorMap *out, const void *w_dev, int type
     return cudaSuccess;
 }
 
-int gemm_token_tile(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 : 128)); }  // with pre-split activations
+int gemm_box_rows(int n) {
+    if (n > kGemmNarrowRows) return gemm_wide_tile(n) / 2;  // either CTA of a pair stages half of a tile
+    return n <= 16 ? 16 : (n <= 32 ? 32 : (n <= 64 ? 64 : 128));
+}
 
-cudaError_t gemm_make_activation_map(GemmTensorMap *out, const void *x16_dev, int64_t row_cap, int64_t cols, int nt) {
-    if (!out || !x16_dev || row_cap <= 0 || cols <= 0 || cols % 64 != 0 || (nt != 16 && nt != 32 && nt != 64 && nt != 128))
+cudaError_t gemm_make_activation_map(GemmTensorMap *out, const void *x16_dev, int64_t row_cap, int64_t cols, int box_rows) {
+    if (!out || !x16_dev || row_cap <= 0 || cols <= 0 || cols % 64 != 0 || box_rows < 16 || box_rows > 128 || box_rows % 16 != 0)
         return cudaErrorInvalidValue;
     typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
@@ -868,7 +871,7 @@ cudaError_t gemm_make_activation_map(GemmTensorMap *out, const void *x16_dev, in
     if (q != cudaDriverEntryPointSuccess || fn == nullptr) return cudaErrorNotSupported;
     const cuuint64_t gdim[2] = {cuuint64_t(cols), cuuint64_t(2 * row_cap)};
     const cuuint64_t gstride[1] = {cuuint64_t(cols) * 2};
-    const cuuint32_t box[2] = {64, cuuint32_t(nt)};  // 64 binary16 = one 128-byte swizzle row
+    const cuuint32_t box[2] = {64, cuuint32_t(box_rows)};  // 64 binary16 = one 128-byte swizzle row
     const cuuint32_t estride[2] = {1, 1};
     CUtensorMap map;
     const CUresult r = reinterpret_cast<EncodeFn>(fn)(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(x16_dev),
@@ -899,7 +902,7 @@ cudaError_t gemm_tc_launch(const GemmArgs &a, cudaStream_t stream) {
             return cudaErrorInvalidValue;
         tiles += (a.seg[s].rows + kTileM - 1) / kTileM;
     }
-    // More than one token tile of pre-split activations: CTA pairs on 256-token tiles (gemm_wide.cu).
+    // More than one token tile of pre-split activations: CTA pairs (gemm_wide.cu).
     if (a.xmap != nullptr && a.n > kGemmNarrowRows) return gemm_wide_launch(a, stream);
     // One arrival counter per output tile: very tall products go in token slabs that fit the counters.
     int slab = a.n;

@@ -12,9 +12,10 @@ struct alignas(64) GemmTensorMap {
 };
 cudaError_t gemm_make_tensor_map(GemmTensorMap *out, const void *w_dev, int type, int64_t rows, int64_t cols);
 // TMA descriptor of a pre-split activation buffer: binary16 [2 * row_cap][cols] (the hi rows, then
-// the lo rows), fetched in swizzled boxes of nt rows x 64 columns; nt is 16, 32, 64 or 128.
-cudaError_t gemm_make_activation_map(GemmTensorMap *out, const void *x16_dev, int64_t row_cap, int64_t cols, int nt);
-int gemm_token_tile(int n);  // the nt the kernel will use for n rows
+// the lo rows), fetched in swizzled boxes of box_rows rows x 64 columns, box_rows from gemm_box_rows.
+cudaError_t gemm_make_activation_map(GemmTensorMap *out, const void *x16_dev, int64_t row_cap, int64_t cols, int box_rows);
+int gemm_box_rows(int n);  // the box of the kernel that takes n rows: its token tile, or half of it on CTA pairs
+constexpr int kGemmBoxes[] = {16, 32, 64, 128, 96};  // every value it returns
 
 struct GemmSeg {
     const uint8_t *w;  // device, GGUF block layout, rows x cols
@@ -51,9 +52,9 @@ struct GemmArgs {
 // Sets the shared-memory attribute of every instantiation (call once, outside stream capture).
 cudaError_t gemm_tc_configure();
 cudaError_t gemm_tc_launch(const GemmArgs &args, cudaStream_t stream);
-// The CTA-pair kernel behind gemm_tc_launch for more than kGemmNarrowRows rows of pre-split activations; the
-// activation map is the one for 128-row boxes.
+// The CTA-pair kernel behind gemm_tc_launch for more than kGemmNarrowRows rows of pre-split activations.
 constexpr int kGemmNarrowRows = 128;
+int gemm_wide_tile(int n);  // its tokens per tile
 cudaError_t gemm_wide_configure();
 cudaError_t gemm_wide_launch(const GemmArgs &args, cudaStream_t stream);
 cudaError_t gemm_trace_bind(unsigned long long *buf, unsigned cap, int mode);

@@ -62,7 +62,7 @@ def test_wide_activations_do_not_overflow_fp16(dev, oracle):
 
 
 def test_tall_product(dev, oracle):
-    """The most weight rows against more than a thousand activation rows: 501 row tiles by five token tiles in one launch, an
+    """The most weight rows against more than a thousand activation rows: 501 row tiles by six token tiles in one launch, an
     arrival counter for either CTA of each. (Without the workspace of the split activations the same product goes in token
     slabs: test_wide_product_inside_a_capture.)"""
     rows, cols, n, t = 128256, 256, 1100, GGMLType.Q4_0
@@ -94,13 +94,13 @@ def test_widest_sweep_batch(dev, oracle, t):
 
 @pytest.mark.parametrize("t", FORMATS + [GGMLType.Q4_1, GGMLType.Q5_K, GGMLType.Q6_K])
 @pytest.mark.parametrize("rows,cols,n", [(100, 256, 129),     # one tile, half of it (and most of the token half) empty
-                                         (256, 512, 256),     # exactly one tile
+                                         (256, 512, 256),     # exactly one tile of 256 tokens
                                          (300, 2048, 257),    # a second row tile and a second token tile of one row
-                                         (1536, 4096, 470),   # 12 tiles on 74 CTA pairs: several pairs per tile
-                                         (6144, 1024, 513),   # 72 tiles: ranges aligned to tiles
+                                         (1536, 4096, 470),   # 18 tiles on 74 CTA pairs: several pairs per tile
+                                         (6144, 1024, 513),   # 72 tiles on 72 pairs: ranges aligned to tiles
                                          (12900, 512, 300)])  # 102 tiles: ranges end inside tiles
 def test_wide_products_on_cta_pairs(dev, oracle, t, rows, cols, n):
-    """More than 128 rows: 256 x 256 tiles on CTA pairs. Same operands as the narrow kernel (weights rounded once to
+    """More than 128 rows: tiles of 256 weight rows on CTA pairs. Same operands as the narrow kernel (weights rounded once to
     binary16, 2^-12 relative on average; activations in 22 bits), so the same expected error."""
     make = jl.synth_tensor if t in FORMATS else jl.random_blocks
     w = make(t, rows * cols, seed=rows + cols + n)
@@ -114,12 +114,35 @@ def test_wide_products_on_cta_pairs(dev, oracle, t, rows, cols, n):
     assert np.array_equal(dev.matmul(t, w, rows, cols, x), got)  # partial tiles are added in a fixed order
 
 
+@pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q8_0])
+@pytest.mark.parametrize("n", [191, 192,        # one tile of 192 tokens
+                               193, 255, 256,   # one tile of 256, in two passes
+                               257, 384, 385,   # tiles of 192 again
+                               576, 577])
+def test_wide_products_over_the_tile_widths(dev, oracle, t, n):
+    """Rows on either side of every token-tile edge and of the CTAs' halves of the tiles, in both forms of the CTA-pair
+    kernel; 300 weight rows (a half-empty row tile) and 2048 columns (32 operand stages: several rounds of every ring)."""
+    rows, cols = 300, 2048
+    w = jl.synth_tensor(t, rows * cols, seed=n)
+    x = np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)
+    got = dev.matmul(t, w, rows, cols, x)
+    half = 128 if 192 < n <= 256 else 96
+    edges = [e for k in range(half, n, half) for e in (k - 1, k)]
+    sample = sorted({0, n - 1, *edges} & set(range(n)))
+    want = oracle.matmul(t, w, x[sample], rows, cols)
+    err = np.linalg.norm(got[sample] - want, axis=1) / np.linalg.norm(want, axis=1)
+    assert err.max() < EXPECT, err
+    assert np.all(np.isfinite(got))
+    assert np.array_equal(dev.matmul(t, w, rows, cols, x), got)
+
+
 def test_wide_product_is_as_close_to_64_bits_as_the_narrow_one(dev):
     """The same rows through the 128-row kernel (an accumulator for either part of the activations) and, as part of a
     wider block, through the CTA pairs. The weights are whole multiples of 2^-7, exact in binary16, so what is left is the
     activations' 22 bits and the binary32 sums: 256 steps over 4096 columns that are cut off at the accumulator's last
-    place, 256 * 2^-24 = 1.5e-5 at most. 148 row tiles of 128 and 74 of 256: every sum runs over whole rows in both."""
-    rows, cols, n = 148 * 128, 4096, 256
+    place, 256 * 2^-24 = 1.5e-5 at most. 148 row tiles of 128 and 74 of 256: every sum runs over whole rows, also in the form that walks a tile twice (256 rows)
+    and in the one with two accumulators (384)."""
+    rows, cols, n = 148 * 128, 4096, 384
     rng = np.random.default_rng(3)
     q = rng.integers(-127, 128, size=(rows, cols)).astype(np.int8)
     blocks = np.empty((rows, cols // 32, 34), np.uint8)
@@ -129,23 +152,23 @@ def test_wide_product_is_as_close_to_64_bits_as_the_narrow_one(dev):
     pick = np.sort(rng.choice(rows, 256, replace=False))
     want = x.astype(np.float64) @ (q[pick].astype(np.float64) * 2.0 ** -7).T
     err = {}
-    for m in (128, n):
+    for m in (128, 256, n):
         got = dev.matmul(GGMLType.Q8_0, blocks.reshape(-1), rows, cols, x[:m])[:, pick]
         err[m] = np.linalg.norm(got[:128] - want[:128]) / np.linalg.norm(want[:128])
-    assert err[n] < 256 * 2.0 ** -24, err
-    assert err[n] <= 1.05 * err[128], err
+    assert max(err.values()) < 256 * 2.0 ** -24, err
+    assert max(err.values()) <= 1.05 * err[128], err
 
 
 @pytest.mark.parametrize("t", [GGMLType.Q4_K, GGMLType.Q8_0])
 @pytest.mark.parametrize("tail", [9, 33, 100, 300])  # a second slab for the 16-, 64- and 128-row kernels and the CTA pairs
 def test_wide_product_in_two_slabs(dev, oracle, t, tail):
-    """14336 columns: 1024 rows of split activations fill the workspace, the rest go in a second slab with a descriptor of
+    """14336 columns: 1152 rows of split activations fill the workspace, the rest go in a second slab with a descriptor of
     its own, behind the first slab's product on the same buffer."""
-    rows, cols, n = 300, 14336, 1024 + tail
+    rows, cols, n = 300, 14336, 1152 + tail
     w = jl.synth_tensor(t, rows * cols, seed=tail)
     x = np.random.default_rng(tail).standard_normal((n, cols)).astype(np.float32)
     got = dev.matmul(t, w, rows, cols, x)
-    sample = [0, 255, 256, 1022, 1023, 1024, 1025, n - 2, n - 1]
+    sample = [0, 191, 192, 1150, 1151, 1152, 1153, n - 2, n - 1]
     want = oracle.matmul(t, w, x[sample], rows, cols)
     err = np.linalg.norm(got[sample] - want, axis=1) / np.linalg.norm(want, axis=1)
     assert err.max() < EXPECT, err
