@@ -382,11 +382,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // converged (one elected lane issues), so every operand is warp-uniform.
         {
             constexpr uint32_t idesc = instr_desc_f16(2 * NT);
-            constexpr uint32_t desc_hi = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);  // SBO, version, 128-byte swizzle
             constexpr uint32_t b_step = uint32_t(S::b_stage >> 4);
             constexpr int kAtom = S::b_sub >> 4;  // descriptor step between the two 64-column atoms
             const uint32_t a_col0 = tmem_d + TmemPlan<NT>::a_stage0;
-            const uint32_t b_lo0 = ((smem_u32(base + S::b_off) >> 4) & 0x3FFFu) | (1u << 16);
+            const uint32_t b_lo0 = sw128_desc_lo(smem_u32(base + S::b_off));
             const uint32_t full0 = smem_u32(a_full), free0 = smem_u32(a_free), acc_full_u32 = smem_u32(acc_full);
             int s = 0, done = 0;
 #ifdef JL_TRACE_EVENTS
@@ -419,7 +418,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
                     __syncwarp();  // elect.sync below names every lane
                     tc_fence_after();
                     umma_stage_f16_tmem_a<2, 4, 6, kAtom, kAtom + 2, kAtom + 4, kAtom + 6>(
-                        tmem_d, a_col, b_lo, desc_hi, idesc, free0 + 8u * uint32_t(s), k == 0 ? 0u : 1u);
+                        tmem_d, a_col, b_lo, kSw128DescHi, idesc, free0 + 8u * uint32_t(s), k == 0 ? 0u : 1u);
                     SLOG(256 + (qlog - 8) * 2 + 1, lane == 0 && qlog >= 8 && qlog < 24);
 #ifdef JL_TRACE_EVENTS
                     ++qlog;

@@ -91,6 +91,8 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // units, bit 16 the (unused) leading byte offset; high word: bits 0-13 the stride between 8-row
 // groups in 16-byte units (1024 >> 4), bit 14 the descriptor version for sm_100, bits 29-31 the
 // swizzle mode (2 = 128 bytes). The issuing thread keeps the low word as a running value.
+constexpr uint32_t kSw128DescHi = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t smem_addr) { return ((smem_addr >> 4) & 0x3FFFu) | (1u << 16); }
 // 16-byte chunk c of row r inside a [rows][64 fp16] swizzled tile.
 __device__ __forceinline__ uint32_t sw128_offset(int r, int c) { return uint32_t(r) * 128u + uint32_t((c ^ (r & 7)) << 4); }
 

@@ -2,9 +2,10 @@
 // products): Y[n][rows] = X[n][cols] . W[rows][cols]^T on CTA pairs, same operands as gemm_tc.cu (weights rounded
 // once to binary16 by the same code, activations as binary16 hi + lo parts, binary32 accumulation).
 //
-// What bounds it: converting the weights, once per token tile, and then the read-out of the tile. A tile is 256 weight rows
-// on two SMs (cta_group::2, M = 256): each CTA converts its own 128 rows into its own tensor memory and stages one half of the
-// tokens, which both tensor cores read.
+// What bounds it: the tensor pipe (ncu: 73 % active in the 8B gate/up launch of 512 rows, issue slots 41 %), the rest the
+// start and the reading out of tiles, which nothing hides. A tile is 256 weight rows on two SMs (cta_group::2, M = 256):
+// each CTA converts its own 128 rows into its own tensor memory and stages one half of the tokens, which both tensor cores
+// read. Against 128 tokens converting a stage takes about as long as multiplying by it.
 //
 // The tensor core cuts every addition off at the accumulator's last place. Lo products (2^-11 of the hi ones) added into the
 // hi sum lose those bits and cut it off twice as often: side by side in one accumulator of 256 tokens, a product of 4096
@@ -203,16 +204,17 @@ template <int NT>
 __device__ __forceinline__ void load_sum(uint32_t acc, int c0, float (&v)[16]) {
     __syncwarp();
     tmem_ld16(acc + uint32_t(c0), v);
-    if (WideForm<NT>::passes == 2) return;
+    if constexpr (WideForm<NT>::passes == 1) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        uint32_t lo[8];
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                     : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3]), "=r"(lo[4]), "=r"(lo[5]), "=r"(lo[6]), "=r"(lo[7])
-                     : "r"(acc + uint32_t(NT + c0 + 8 * h)));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        for (int h = 0; h < 2; ++h) {
+            uint32_t lo[8];
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                         : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3]), "=r"(lo[4]), "=r"(lo[5]), "=r"(lo[6]), "=r"(lo[7])
+                         : "r"(acc + uint32_t(NT + c0 + 8 * h)));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[8 * h + j] += __uint_as_float(lo[j]);
+            for (int j = 0; j < 8; ++j) v[8 * h + j] += __uint_as_float(lo[j]);
+        }
     }
 }
 
@@ -430,8 +432,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
     } else if (warp == kEpiWarps + kConvWarps) {
         // ---- tensor-core issue (first CTA of the pair) -----------------------------------------------------
         if (rank == 0) {
-            constexpr uint32_t desc_hi = uint32_t(1024 >> 4) | (1u << 14) | (2u << 29);  // SBO, version, 128-byte swizzle
-            const uint32_t b_lo0 = ((smem_u32(base) >> 4) & 0x3FFFu) | (1u << 16);
+            const uint32_t b_lo0 = sw128_desc_lo(smem_u32(base));
             const uint32_t a_full0 = smem_u32(a_full), done0 = smem_u32(done), b_full0 = smem_u32(b_full);
             int st = 0, turn = 0, issued = 0;
             uint32_t par = 0;
@@ -449,7 +450,7 @@ __global__ void __launch_bounds__(kWideThreads, 1)
                     }
                     tc_fence_after();
                     umma_stage_pair<NT>(tmem_d, tmem_d + uint32_t(F::acc_cols) + uint32_t(st) * kAStageCols,
-                                        b_lo0 + uint32_t(st) * uint32_t(F::b_stage >> 4), desc_hi, done0 + 8u * uint32_t(st),
+                                        b_lo0 + uint32_t(st) * uint32_t(F::b_stage >> 4), kSw128DescHi, done0 + 8u * uint32_t(st),
                                         k == 0 ? 0u : 1u);
                     ++issued;
                     if (++st == AS) {
