@@ -20,7 +20,7 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB = PKG / "lib"
 
-CUDA_SOURCES = ["gemv.cu", "ops.cu", "engine.cu", "static_entry.cu", "gemm_tc.cu", "gemm_wide.cu", "attn_prompt_tc.cu", "tp_exchange.cu", "gguf_loader.cu",
+CUDA_SOURCES = ["gemv.cu", "ops.cu", "attn_split.cu", "engine.cu", "static_entry.cu", "gemm_tc.cu", "gemm_wide.cu", "attn_prompt_tc.cu", "tp_exchange.cu", "gguf_loader.cu",
                 "sampler.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

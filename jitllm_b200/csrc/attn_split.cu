@@ -1,0 +1,502 @@
+// RoPE + KV append + paged decode attention with the keys of a sequence split over CTAs (sm_100a), for launches that have
+// fewer (row, KV head) pairs than the GPU has room for.
+//
+// What it computes: CpuOperations.rope + appendKeyValue + attention (inference/op/CpuOperations.java:94-204), softmax online;
+// K and V are rounded to binary16 on append exactly as ArrayHalfFloatTensor.setFloat does
+// (tensor/standard/ArrayHalfFloatTensor.java:33-40).
+//
+// One CTA of eight warps = (range of keys, KV head, row). The G query heads that share the KV head are rows of one MMA
+// tile: a query, and a probability, is the exact sum of three binary16 parts, which are three rows each (3 G <= 12 of the 16
+// rows; G = 8 takes two tiles), so q.k and p.v keep their 32 bits while keys and values are binary16 as stored. Tiles of 64
+// keys come through a double buffer by cp.async; warp w multiplies sixteen of a tile's keys and half of the output dimensions.
+// A launch is latency: 64 keys per CTA as long as there are CTAs, then longer ranges. The last CTA of a (row, KV head) to
+// finish folds the ranges' results; the arrival is one atomic. The kernel before this one took scalar products (8 keys per
+// warp in 1.2 us) and folded sixteen warps and a cluster of eight CTAs (2.5 us).
+#include "ops.cuh"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+namespace jl {
+
+JL_TRACE_DEFINE_BIND(attn_split_trace_bind)
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kTile = 64;         // keys
+constexpr int kGroups = kTile / 16;
+constexpr int kKeysPerSplit = 64;
+constexpr int kPages = 512;       // page numbers kept in shared memory
+
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
+// x as the sum of three binary16 values of eight significant bits each: all 24 of it. (Not of eleven: the tensor core cuts its
+// sums of sixteen products off at some 2^-24 of the largest, and a part's products with binary16 keys would reach below that.
+// Eight bits leave the first part's sums whole, and what is cut off the other two is 2^-8 and 2^-16 of it.)
+__device__ __forceinline__ void split3(float x, __half (&h)[3]) {
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const float part = __bfloat162float(__float2bfloat16_rn(x));
+        h[p] = __float2half_rn(part);
+        x -= part;
+    }
+    h[2] = __float2half_rn(x);
+}
+
+template <int HD, int G>
+struct SplitAttn {
+    static constexpr int LD = HD + 8;          // halves per row: no bank conflicts
+    static constexpr int QT = G == 8 ? 2 : 1;  // sixteen-row tiles that hold three parts of G heads
+    struct Smem {
+        alignas(16) __half q[QT * 16][LD];
+        int pages[kPages];
+        float w[kGroups][G];  // merge weights
+        float inv[G], sum[G], top[G];
+        int is_last;
+        union {
+            struct {
+                alignas(16) __half k[2][kTile][LD];
+                alignas(16) __half v[2][kTile][LD];
+            } tile;
+            float merge[kGroups][G][HD + 2];
+            float fold[1024];  // [range][head] maxima, then weights
+        };
+    };
+};
+
+template <int HD, int G>
+__global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs a) {
+    using A = SplitAttn<HD, G>;
+    constexpr int LD = A::LD, QT = A::QT, DB = HD / 16, ROW = HD + 2, PARTS = HD / 8;
+    extern __shared__ __align__(16) uint8_t smem_raw[];
+    typename A::Smem &sm = *reinterpret_cast<typename A::Smem *>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int split = blockIdx.x, kvh = blockIdx.y, b = blockIdx.z;
+    const int trace = trace_begin(kTraceAttn);
+    pdl_launch_dependents();
+    const bool on = a.active == nullptr || a.active[b] != 0;
+    const bool dec = a.append != 0;
+    // A decode launch reads what no kernel of this step writes (position, slot, page table, old keys) before it waits for
+    // the one that produces q, k and v: positions and slots are written by the host or by advance_kernel, and the kernel
+    // after that one releases its dependents only when it has waited itself. The rows of a prompt wait first: their keys
+    // were appended by the kernel ahead.
+    if (!dec) pdl_wait();
+    const int pos = on ? a.positions[b] : 0, slot = on ? a.slots[b] : 0;
+    const int old = dec ? pos : pos + 1;  // keys in the pages
+    const int nsplit = max(1, min(a.nsplit, (old + kKeysPerSplit - 1) / kKeysPerSplit));
+    if (!on || split >= nsplit) {
+        if (dec) pdl_wait();
+        return;
+    }
+    const int chunk = (old + nsplit - 1) / nsplit;
+    const int start = min(old, split * chunk), stop = min(old, start + chunk);
+    const bool owns_new = dec && split == nsplit - 1;  // this step's own key and value: behind the last range
+    const int end = stop + (owns_new ? 1 : 0);
+    const int bt = a.kv.block_tokens, kv_dim = a.kv.kv_dim;
+    const int64_t block_stride = int64_t(a.kv.layers) * bt * kv_dim, in_layer = int64_t(a.layer) * bt * kv_dim + int64_t(kvh) * HD;
+    const int32_t *table = a.kv.block_table + int64_t(slot) * a.kv.blocks_per_slot;
+    const int first_page = start / bt, npages = stop > start ? (stop - 1) / bt - first_page + 1 : 0;
+    for (int i = tid; i < min(npages, kPages); i += kThreads) sm.pages[i] = table[first_page + i];
+    for (int i = tid; i < QT * 16 * LD / 2; i += kThreads) reinterpret_cast<uint32_t *>(&sm.q[0][0])[i] = 0u;
+    constexpr int kPairs = (G + 2) * (HD / 2), kRounds = (kPairs + kThreads - 1) / kThreads;
+    float cr[kRounds], ci[kRounds];  // of this thread's pairs of dimensions
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int i = (tid + r * kThreads) % (HD / 2);
+        cr[r] = a.rope_cos[size_t(pos) * (HD / 2) + i];
+        ci[r] = a.rope_sin[size_t(pos) * (HD / 2) + i];
+    }
+    __syncthreads();
+    const uint32_t k0 = smem_u32(&sm.tile.k[0][0][0]), v0 = smem_u32(&sm.tile.v[0][0][0]);
+    auto load = [&](int t0, int buf) {
+#pragma unroll
+        for (int i = 0; i < kTile * PARTS / kThreads; ++i) {
+            const int key = (i * kThreads + tid) / PARTS, part = tid % PARTS, t = t0 + key;
+            const uint32_t at = uint32_t((buf * kTile + key) * LD + part * 8) * 2;
+            if (t < stop) {
+                const int pg = t / bt, in = pg - first_page;
+                const int64_t off = int64_t(in < kPages ? sm.pages[in] : table[pg]) * block_stride + in_layer + int64_t(t - pg * bt) * kv_dim + part * 8;
+                cp_async16(k0 + at, a.kv.kpool + off);
+                cp_async16(v0 + at, a.kv.vpool + off);
+            } else {
+                sts64(k0 + at, 0u, 0u);
+                sts64(k0 + at + 8, 0u, 0u);
+                sts64(v0 + at, 0u, 0u);
+                sts64(v0 + at + 8, 0u, 0u);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(start, 0);
+    if (dec) pdl_wait();
+    trace_mark(trace, 2);
+    trace_word(trace, 6, trace_latest_exit());
+    // Queries rotated, and the new key and value: rotated, rounded to binary16 as the append does.
+    float qx[kRounds] = {}, qy[kRounds] = {};
+    uint32_t fresh[kRounds] = {};
+    bool large = false;
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int idx = tid + r * kThreads, i = idx % (HD / 2);
+        if (idx < G * (HD / 2)) {
+            const float2 x = __ldcg(reinterpret_cast<const float2 *>(a.q + size_t(b) * a.dim + size_t(kvh * G + idx / (HD / 2)) * HD) + i);
+            qx[r] = __fsub_rn(__fmul_rn(x.x, cr[r]), __fmul_rn(x.y, ci[r]));
+            qy[r] = __fadd_rn(__fmul_rn(x.x, ci[r]), __fmul_rn(x.y, cr[r]));
+            large = large || fmaxf(fabsf(qx[r]), fabsf(qy[r])) > 32768.0f;
+        } else if (owns_new && idx < kPairs) {
+            const bool is_k = idx < (G + 1) * (HD / 2);
+            const float2 x = __ldcg(reinterpret_cast<const float2 *>((is_k ? a.k : a.v) + size_t(b) * kv_dim + size_t(kvh) * HD) + i);
+            const __half2 h = is_k ? __halves2half2(__float2half_rn(__fsub_rn(__fmul_rn(x.x, cr[r]), __fmul_rn(x.y, ci[r]))),
+                                                    __float2half_rn(__fadd_rn(__fmul_rn(x.x, ci[r]), __fmul_rn(x.y, cr[r]))))
+                                   : __halves2half2(__float2half_rn(x.x), __float2half_rn(x.y));
+            const int64_t off = int64_t(table[pos / bt]) * block_stride + in_layer + int64_t(pos % bt) * kv_dim;
+            *reinterpret_cast<__half2 *>((is_k ? a.kv.kpool : a.kv.vpool) + off + 2 * i) = h;
+            fresh[r] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
+    // Queries beyond the range of binary16 are scaled by a power of two (the same for all ranges: they see the same queries).
+    float q_scale = 1.0f;
+    if (__syncthreads_or(large)) {
+        if (tid == 0) sm.is_last = 0;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kRounds; ++r) {
+            const float most = fmaxf(fabsf(qx[r]), fabsf(qy[r]));
+            if (most < INFINITY) atomicMax(&sm.is_last, __float_as_int(most));
+        }
+        __syncthreads();
+        q_scale = exp2f(static_cast<float>(14 - ((sm.is_last >> 23) - 127)));
+    }
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+        const int idx = tid + r * kThreads, i = idx % (HD / 2);
+        if (idx < G * (HD / 2)) {
+            const int g = idx / (HD / 2);
+            __half p0[3], p1[3];
+            split3(qx[r] * q_scale, p0);
+            split3(qy[r] * q_scale, p1);
+#pragma unroll
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<__half2 *>(&sm.q[p * G + g][2 * i]) = __halves2half2(p0[p], p1[p]);
+        }
+    }
+    trace_mark(trace, 3);
+    const float inv_sqrt = 1.0f / sqrtf(static_cast<float>(HD)), unscale = 1.0f / q_scale;
+    const int gl = lane >> 2, t = lane & 3, kg = warp & (kGroups - 1), half = warp / kGroups;
+    constexpr float kUp = 4096.0f;  // probabilities are split as multiples of 2^-12: the small ones' parts stay normal
+    float m = -INFINITY, l = 0.f, o[DB][4];
+#pragma unroll
+    for (int d = 0; d < DB; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
+    // sum over the parts of a head: the lanes whose rows have the same head
+    auto join = [&](float x) {
+#pragma unroll
+        for (int s = 4 * G; s < 32; s *= 2) x += __shfl_xor_sync(0xffffffffu, x, s);
+        return x;
+    };
+    for (int t0 = start, buf = 0; t0 < end; t0 += kTile, buf ^= 1) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the tile is there, and everybody is done with the other buffer
+        if (t0 + kTile < end) load(t0 + kTile, buf ^ 1);
+        if (owns_new && end - 1 - t0 < kTile) {  // the new key's tile
+#pragma unroll
+            for (int r = 0; r < kRounds; ++r) {
+                const int idx = tid + r * kThreads, i = idx % (HD / 2);
+                if (idx >= G * (HD / 2) && idx < kPairs) {
+                    const bool is_k = idx < (G + 1) * (HD / 2);
+                    *reinterpret_cast<uint32_t *>(is_k ? &sm.tile.k[buf][pos - t0][2 * i] : &sm.tile.v[buf][pos - t0][2 * i]) = fresh[r];
+                }
+            }
+            __syncthreads();
+        }
+        const int key0 = 16 * kg;
+        if (t0 + key0 >= end) continue;
+        // Every product has an accumulator of its own and is added by the rounding adder, pairs of pairs: the tensor core cuts
+        // additions off.
+        float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f}, level[2][8];
+        const uint32_t qa = smem_u32(&sm.q[0][0]) + uint32_t((lane & 15) * LD + (lane >> 4) * 8) * 2;
+        const uint32_t ka = k0 + uint32_t((buf * kTile + key0 + (lane & 7) + ((lane >> 4) & 1) * 8) * LD + ((lane >> 3) & 1) * 8) * 2;
+#pragma unroll
+        for (int ks = 0; ks < HD / 16; ++ks) {
+            uint32_t qf[4], kf[4];
+            ldmatrix4(qf, qa + ks * 32);
+            ldmatrix4(kf, ka + ks * 32);
+            float x0[4] = {0.f, 0.f, 0.f, 0.f}, x1[4] = {0.f, 0.f, 0.f, 0.f};
+            mma_f16(x0, qf, kf[0], kf[1]);
+            mma_f16(x1, qf, kf[2], kf[3]);
+            if constexpr (QT == 2) {  // the third parts, rows 0-7 of the second tile
+                uint32_t ql[4];
+                float y0[4] = {0.f, 0.f, 0.f, 0.f}, y1[4] = {0.f, 0.f, 0.f, 0.f};
+                ldmatrix4(ql, qa + uint32_t(16 * LD * 2) + ks * 32);
+                mma_f16(y0, ql, kf[0], kf[1]);
+                mma_f16(y1, ql, kf[2], kf[3]);
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    x0[2 + e] += y0[e];
+                    x1[2 + e] += y1[e];
+                }
+            }
+            // x = the sum of a whole block of 2^n steps: up the tree as long as its partner waits there
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                float x = x0[e], y = x1[e];
+                if ((ks & 1) != 0) {
+                    x += level[0][e];
+                    y += level[0][4 + e];
+                    if ((ks & 2) != 0) {
+                        s0[e] += x + level[1][e];
+                        s1[e] += y + level[1][4 + e];
+                    } else {
+                        level[1][e] = x;
+                        level[1][4 + e] = y;
+                    }
+                } else {
+                    level[0][e] = x;
+                    level[0][4 + e] = y;
+                }
+            }
+        }
+        // this lane: head gl % G against keys 2t, 2t + 1 of either eight
+        float s[4] = {join(s0[0] + s0[2]), join(s0[1] + s0[3]), join(s1[0] + s1[2]), join(s1[1] + s1[3])};
+        float top = -INFINITY;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int key = t0 + key0 + (c >> 1) * 8 + 2 * t + (c & 1);
+            s[c] = key < end ? s[c] * unscale * inv_sqrt : -INFINITY;
+            top = fmaxf(top, s[c]);
+        }
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+        const float mn = fmaxf(m, top);
+        // every score of the group may be -inf (an infinite query or key): no weight, as the reference's exp(-inf - max)
+        const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
+        m = mn;
+        l *= corr;
+        uint32_t pf[QT][4];
+        __half part[4][3];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float p = mn == -INFINITY ? 0.f : expf(s[c] - mn);
+            l += p;
+            split3(p * kUp, part[c]);
+        }
+        // rows gl and gl + 8 of the probability tile(s): part row / G of head row % G
+#pragma unroll
+        for (int f = 0; f < 2; ++f) {
+            uint32_t w[3];
+#pragma unroll
+            for (int p = 0; p < 3; ++p) {
+                const __half2 h = __halves2half2(part[2 * f][p], part[2 * f + 1][p]);
+                w[p] = *reinterpret_cast<const uint32_t *>(&h);
+            }
+            const int which = gl / G;
+            if constexpr (G == 8) {
+                pf[0][2 * f] = w[0];
+                pf[0][2 * f + 1] = w[1];
+                pf[QT - 1][2 * f] = w[2];
+                pf[QT - 1][2 * f + 1] = 0u;
+            } else {
+                pf[0][2 * f] = which == 0 ? w[0] : which == 1 ? w[1] : which == 2 ? w[2] : 0u;
+                pf[0][2 * f + 1] = G == 4 && which == 0 ? w[2] : 0u;
+            }
+        }
+        const uint32_t va = v0 + uint32_t((buf * kTile + key0 + (lane & 15)) * LD + half * (HD / 2) + (lane >> 4) * 8) * 2;
+#pragma unroll
+        for (int d = 0; d < DB; d += 2) {
+            uint32_t vf[4];
+            ldmatrix4_trans(vf, va + d * 16);
+            float x0[4] = {0.f, 0.f, 0.f, 0.f}, x1[4] = {0.f, 0.f, 0.f, 0.f};
+            if constexpr (QT == 2) {
+                mma_f16(x0, pf[1], vf[0], vf[1]);
+                mma_f16(x1, pf[1], vf[2], vf[3]);
+            }
+            mma_f16(x0, pf[0], vf[0], vf[1]);
+            mma_f16(x1, pf[0], vf[2], vf[3]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                o[d][e] = fmaf(o[d][e], corr, x0[e]);
+                o[d + 1][e] = fmaf(o[d + 1][e], corr, x1[e]);
+            }
+        }
+    }
+    trace_mark(trace, 4);
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    __syncthreads();  // everybody is done with the tiles: their memory becomes the merge area
+#pragma unroll
+    for (int d = 0; d < DB; ++d) {
+        const float x = join(o[d][0] + o[d][2]), y = join(o[d][1] + o[d][3]);
+        if (gl < G) {
+            sm.merge[kg][gl][half * (HD / 2) + d * 8 + 2 * t] = x * (1.0f / kUp);
+            sm.merge[kg][gl][half * (HD / 2) + d * 8 + 2 * t + 1] = y * (1.0f / kUp);
+        }
+    }
+    if (half == 0 && gl < G && t == 0) {
+        sm.merge[kg][gl][HD] = m;
+        sm.merge[kg][gl][HD + 1] = l;
+    }
+    __syncthreads();
+    if (tid < G * kGroups) {  // four lanes per head: the groups' maxima and sums (one without keys weighs nothing)
+        const int g = tid / kGroups, w = tid % kGroups;
+        const unsigned lanes = G * kGroups >= 32 ? 0xffffffffu : (1u << (G * kGroups)) - 1u;
+        const float mw = sm.merge[w][g][HD];
+        float M = mw;
+#pragma unroll
+        for (int s = 1; s < kGroups; s *= 2) M = fmaxf(M, __shfl_xor_sync(lanes, M, s));
+        const float wgt = mw == -INFINITY ? 0.f : expf(mw - M);
+        float L = sm.merge[w][g][HD + 1] * wgt;
+#pragma unroll
+        for (int s = 1; s < kGroups; s *= 2) L += __shfl_xor_sync(lanes, L, s);
+        sm.w[w][g] = wgt;
+        if (w == 0) {
+            sm.top[g] = M;
+            sm.sum[g] = L;
+        }
+    }
+    __syncthreads();
+    float *parts = a.partial + (size_t(b) * a.kv_heads + kvh) * a.nsplit * (G * ROW);  // [range][head][HD + 2]
+    for (int idx = tid; idx < G * HD; idx += kThreads) {
+        const int g = idx / HD, d = idx - g * HD;
+        float val = 0.f;
+#pragma unroll
+        for (int w = 0; w < kGroups; ++w) val += sm.merge[w][g][d] * sm.w[w][g];
+        if (nsplit == 1) {
+            attn_store(a, size_t(b), (kvh * G + g) * HD + d, val / sm.sum[g]);
+        } else {
+            float *p = parts + (size_t(split) * G + g) * ROW;
+            p[d] = val;
+            if (d == 0) {
+                p[HD] = sm.top[g];
+                p[HD + 1] = sm.sum[g];
+            }
+        }
+    }
+    if (nsplit == 1) {
+        trace_mark(trace, 5);
+        if (tid == 0) trace_cta_exit();
+        return;
+    }
+    // The last range of this (row, KV head) to finish folds them all.
+    __syncthreads();
+    unsigned *arrived = a.counters + size_t(b) * a.kv_heads + kvh;
+    if (tid == 0) {
+        unsigned before;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(before) : "l"(arrived) : "memory");
+        sm.is_last = before == unsigned(nsplit) - 1u;
+    }
+    __syncthreads();
+    if (!sm.is_last) return;
+    for (int idx = tid; idx < G * nsplit; idx += kThreads) sm.fold[idx] = __ldcg(parts + size_t(idx) * ROW + HD);  // [range][head]
+    // this thread's output elements in the first ranges, on their way meanwhile
+    constexpr int kOut = (G * HD + kThreads - 1) / kThreads, kEarly = 4;
+    float mine[kOut][kEarly];
+#pragma unroll
+    for (int r = 0; r < kOut; ++r) {
+        const int idx = tid + r * kThreads;
+#pragma unroll
+        for (int s = 0; s < kEarly; ++s) mine[r][s] = idx < G * HD && s < nsplit ? __ldcg(parts + (size_t(s) * G + idx / HD) * ROW + idx % HD) : 0.f;
+    }
+    __syncthreads();
+    if (warp < G) {
+        float M = -INFINITY;
+        for (int s = lane; s < nsplit; s += 32) M = fmaxf(M, sm.fold[s * G + warp]);
+        M = warp_max(M);
+        float L = 0.f;
+        for (int s = lane; s < nsplit; s += 32) {
+            const float ms = sm.fold[s * G + warp];
+            const float w = ms == -INFINITY ? 0.f : expf(ms - M);
+            sm.fold[s * G + warp] = w;
+            L += __ldcg(parts + (size_t(s) * G + warp) * ROW + HD + 1) * w;
+        }
+        L = warp_sum(L);
+        if (lane == 0) sm.inv[warp] = 1.0f / L;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kOut; ++r) {
+        const int idx = tid + r * kThreads;
+        if (idx >= G * HD) break;
+        const int g = idx / HD, d = idx - g * HD;
+        float val = 0.f;
+#pragma unroll
+        for (int s = 0; s < kEarly; ++s)
+            if (s < nsplit) val += mine[r][s] * sm.fold[s * G + g];
+        for (int s0 = kEarly; s0 < nsplit; s0 += 8) {
+            float more[8];
+#pragma unroll
+            for (int s = 0; s < 8; ++s) more[s] = s0 + s < nsplit ? __ldcg(parts + (size_t(s0 + s) * G + g) * ROW + d) : 0.f;
+#pragma unroll
+            for (int s = 0; s < 8; ++s)
+                if (s0 + s < nsplit) val += more[s] * sm.fold[(s0 + s) * G + g];
+        }
+        attn_store(a, size_t(b), (kvh * G + g) * HD + d, val * sm.inv[g]);
+    }
+    if (tid == 0) {
+        *arrived = 0u;
+        trace_cta_exit();
+    }
+    trace_mark(trace, 5);
+}
+
+template <int HD, int G>
+cudaError_t launch_t(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic) {
+    if (a.nsplit < 1 || a.nsplit * G > 1024) return cudaErrorInvalidValue;  // the fold's table
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.nsplit, a.kv_heads, width);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = sizeof(typename SplitAttn<HD, G>::Smem);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = programmatic ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, attn_split_kernel<HD, G>, a);
+}
+template <int HD>
+cudaError_t launch_hd(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic) {
+    switch (a.heads / a.kv_heads) {
+        case 1: return launch_t<HD, 1>(a, width, stream, programmatic);
+        case 2: return launch_t<HD, 2>(a, width, stream, programmatic);
+        case 4: return launch_t<HD, 4>(a, width, stream, programmatic);
+        case 8: return launch_t<HD, 8>(a, width, stream, programmatic);
+        default: return cudaErrorInvalidValue;
+    }
+}
+template <int HD, int G>
+cudaError_t configure_t() {
+    return cudaFuncSetAttribute(attn_split_kernel<HD, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(typename SplitAttn<HD, G>::Smem)));
+}
+template <int HD>
+cudaError_t configure_hd() {
+    cudaError_t e;
+    if ((e = configure_t<HD, 1>()) != cudaSuccess) return e;
+    if ((e = configure_t<HD, 2>()) != cudaSuccess) return e;
+    if ((e = configure_t<HD, 4>()) != cudaSuccess) return e;
+    return configure_t<HD, 8>();
+}
+
+}  // namespace
+
+cudaError_t attention_split_configure() {
+    const cudaError_t e = configure_hd<128>();
+    return e != cudaSuccess ? e : configure_hd<64>();
+}
+
+cudaError_t attention_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic) {
+    if (a.head_dim == 128) return launch_hd<128>(a, width, stream, programmatic);
+    if (a.head_dim == 64) return launch_hd<64>(a, width, stream, programmatic);
+    return cudaErrorInvalidValue;
+}
+
+}  // namespace jl

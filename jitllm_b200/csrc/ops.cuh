@@ -33,7 +33,22 @@ struct AttnArgs {
     int *status;        // device status word (attention_prompt_launch), nullable
 };
 
+// One attention output element, and its binary16 hi / lo parts at the element's place in the tensor-core
+// path's operand order when the launch asks for them.
+__device__ __forceinline__ void attn_store(const AttnArgs &a, size_t row, int k, float v) {
+    a.out[row * a.dim + k] = v;
+    if (a.out_hi != nullptr) {
+        const int p = (k & ~3) | ((k & 1) << 1) | ((k >> 1) & 1);
+        const __half h = __float2half_rn(v);
+        static_cast<__half *>(a.out_hi)[row * a.dim + p] = h;
+        static_cast<__half *>(a.out_lo)[row * a.dim + p] = __float2half_rn(v - __half2float(h));
+    }
+}
+
 cudaError_t attention_configure();
+cudaError_t attention_split_configure();
+cudaError_t attn_split_trace_bind(unsigned long long *buf, unsigned cap, int mode);
+// The keys of every row split over up to nsplit CTAs (attn_split.cu).
 cudaError_t attention_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic);
 // The rows of one prompt chunk (all of one sequence, their keys already in the pages; append = 0): tiles of 128 rows
 // (heads x tokens) against tiles of 128 keys on the tensor cores (attn_prompt_tc.cu) instead of one walk over the
@@ -44,7 +59,8 @@ cudaError_t attention_prompt_launch(const AttnArgs &a, int n, cudaStream_t strea
 // query heads as the rows of a tensor-core tile; rotates and appends the step's own key and value itself.
 cudaError_t attention_batch_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic);
 size_t attention_partial_floats(int width, int heads, int nsplit, int head_dim);
-// Key-range splits per (row, KV head) for a launch of `width` rows: cluster size times clusters.
+// Key ranges per (row, KV head), at most, for a launch of `width` rows.
+constexpr int kAttnMaxSplits = 20;
 int attention_splits(int sm_count, int width, int kv_heads);
 
 // x[row] = getFloat of embedding row tokens[row] (inference/op/CpuOperations.java:30-32).
