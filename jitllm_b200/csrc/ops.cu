@@ -337,22 +337,29 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
 // One CTA per (batch row, KV head). The G query heads that share the KV head are rows 0..G-1 of the 16-row A
 // operand (the other rows are zero), so the scores of all heads against 64 keys are 16 mma.sync per key tile
 // and warp instead of a few thousand scalar multiply-adds, and the kernel runs at the speed the pages arrive.
-// The four warps share the staged key / value tiles (cp.async, one tile ahead, as in the prompt kernel) and
-// split each tile's 64 keys four ways; each keeps its own running maximum, sum and output, merged at the end.
+// The four warps are independent until the end: of every 64 keys each takes sixteen, stages them in a ring of its
+// own (cp.async, two groups of sixteen ahead) and keeps its own running maximum, sum and output, merged at the end.
+// Nothing but the pages' arrival should bound this kernel, so the instructions beside the products are few: the
+// sixteen keys of a group share a page whenever the page size is a multiple of sixteen, and then one page lookup and
+// one pointer serve all of a lane's copies of the group; no barrier of the CTA stands between two groups. (With
+// tiles of 64 keys staged by the whole CTA, every key divided by the page size for its own address and two barriers
+// a tile, a step of the 8B shape took 4519 us with 32 rows of 256-768 keys, now 4210: 9.7 us less in each of 32 launches;
+// with 64 rows of 210-630 keys the gain is the same.)
 // The step's own key and value (rotated, rounded to binary16 as the append does) are written to the page and
-// dropped into the staged tile by the CTA itself, so nothing else has to run before it.
+// dropped into the staged group by the warp that holds it, so nothing else has to run before it.
 // Arithmetic: inference/op/CpuOperations.java:94-235, as attn_split.cu.
 template <int HD, int G>
 struct BatchAttnShape {
     static constexpr int warps = 4;
-    static constexpr int tk = 64;       // keys per tile: sixteen per warp
-    static constexpr int depth = 3;     // tile buffers: two tiles in flight while one is used
+    static constexpr int tk = 16;       // keys per group, the depth of one MMA of the value product
+    static constexpr int depth = 3;     // group buffers per warp: two groups in flight while one is used
     static constexpr int ld = HD + 8;
     static constexpr int pages = 256;   // page bases kept in shared memory (4 K keys of 16-token pages)
     static constexpr int tile_halves = tk * ld;
     static constexpr int merge_floats = warps * G * (HD + 2);  // overlays the tiles once the keys are done
-    static constexpr int smem_bytes = depth * 2 * tile_halves * 2 + pages * 8;  // two CTAs per SM at HD = 128
-    static_assert(merge_floats * 4 <= depth * 2 * tile_halves * 2, "the merge area overlays the tile buffers");
+    static constexpr int ring_bytes = warps * depth * 2 * tile_halves * 2;
+    static constexpr int smem_bytes = ring_bytes + pages * 8;  // two CTAs per SM at HD = 128
+    static_assert(merge_floats * 4 <= ring_bytes, "the merge area overlays the rings");
 };
 
 template <int HD, int G>
@@ -360,13 +367,13 @@ __global__ void __launch_bounds__(BatchAttnShape<HD, G>::warps * 32, 2)
     attn_batch_kernel(const AttnArgs a) {
     using P = BatchAttnShape<HD, G>;
     constexpr int TK = P::tk, LD = P::ld, KS = HD / 16, DB = HD / 8, NBUF = P::depth;
-    constexpr int PARTS = HD / 8;                       // 16-byte chunks per key row
-    constexpr int KEYS_PER_PASS = P::warps * 32 / PARTS;  // key rows one pass of the CTA's threads covers
+    constexpr int PARTS = HD / 8;               // 16-byte chunks per key row
+    constexpr int KEYS_PER_PASS = 32 / PARTS;   // key rows one pass of a warp's lanes covers
     extern __shared__ __align__(16) uint8_t batch_smem[];
-    __half *tiles = reinterpret_cast<__half *>(batch_smem);  // [buffer][K | V][TK][LD]
-    int64_t *page_base = reinterpret_cast<int64_t *>(batch_smem + NBUF * 2 * P::tile_halves * 2);
-    float *merge = reinterpret_cast<float *>(batch_smem);  // after the last tile
+    int64_t *page_base = reinterpret_cast<int64_t *>(batch_smem + P::ring_bytes);
+    float *merge = reinterpret_cast<float *>(batch_smem);  // after the last group
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __half *ring = reinterpret_cast<__half *>(batch_smem) + warp * NBUF * 2 * P::tile_halves;  // [buffer][K | V][TK][LD]
     const int kvh = blockIdx.x, b = blockIdx.y;
     const int qr = lane >> 2, qc = lane & 3;
     const bool on = a.active == nullptr || a.active[b] != 0;
@@ -384,38 +391,56 @@ __global__ void __launch_bounds__(BatchAttnShape<HD, G>::warps * 32, 2)
         }
     }
     __syncthreads();
-    const uint32_t tiles_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(tiles));
+    const uint32_t ring_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
     auto key_offset = [&](int t) -> int64_t {
         const int pg = t / bt;
         const int64_t base = pg < P::pages ? page_base[pg] : kv_offset(a.kv, slot, t - t % bt, a.layer) + int64_t(kvh) * HD;
         return base + int64_t(t % bt) * a.kv.kv_dim;
     };
-    // Keys 0 .. pos - 1 come from the pages (this step's key, position pos, is written below). A thread copies the
-    // same 16-byte part of every KEYS_PER_PASS-th key row, of the key tile and of the value tile.
-    const int part = tid % PARTS, key_first = tid / PARTS;
-    auto stage = [&](int t0, int buf) {
+    // Group g of this warp: keys first_key + 64 g .. + 15. Keys 0 .. pos - 1 come from the pages (this step's key,
+    // position pos, is written below); a lane copies the same 16-byte part of every KEYS_PER_PASS-th key row.
+    constexpr int STRIDE = P::warps * TK;
+    const int first_key = warp * TK;
+    const int part = lane % PARTS, key_first = lane / PARTS;
+    const bool one_page = bt % TK == 0;  // the sixteen keys of every group lie in one page
+    auto stage = [&](int g, int buf) {
+        const int t0 = first_key + g * STRIDE;
+        const uint32_t dst = ring_u32 + uint32_t(((buf * 2) * P::tile_halves + key_first * LD + part * 8) * 2);
+        constexpr uint32_t V = uint32_t(P::tile_halves * 2);
+        if (one_page && t0 + TK <= pos) {
+            const int64_t off = key_offset(t0) + int64_t(key_first) * a.kv.kv_dim + part * 8;
+            const __half *ks = a.kv.kpool + off, *vs = a.kv.vpool + off;
+            const int step = KEYS_PER_PASS * a.kv.kv_dim;
 #pragma unroll
-        for (int key = key_first; key < TK; key += KEYS_PER_PASS) {
-            const uint32_t dk = tiles_u32 + uint32_t(((buf * 2) * P::tile_halves + key * LD + part * 8) * 2);
-            const uint32_t dv = dk + uint32_t(P::tile_halves * 2);
-            const int t = t0 + key;
-            if (t < pos) {
-                const int64_t off = key_offset(t) + part * 8;
-                cp_async_16(dk, a.kv.kpool + off);
-                cp_async_16(dv, a.kv.vpool + off);
-            } else {
-                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dk), "r"(0u) : "memory");
-                asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dv), "r"(0u) : "memory");
+            for (int i = 0; i < TK / KEYS_PER_PASS; ++i) {
+                cp_async_16(dst + uint32_t(i * KEYS_PER_PASS * LD * 2), ks);
+                cp_async_16(dst + V + uint32_t(i * KEYS_PER_PASS * LD * 2), vs);
+                ks += step;
+                vs += step;
+            }
+        } else {  // a page size that is no multiple of sixteen, or the last keys
+#pragma unroll 1
+            for (int i = 0; i < TK / KEYS_PER_PASS; ++i) {
+                const uint32_t dk = dst + uint32_t(i * KEYS_PER_PASS * LD * 2);
+                const int t = t0 + key_first + i * KEYS_PER_PASS;
+                if (t < pos) {
+                    const int64_t off = key_offset(t) + part * 8;
+                    cp_async_16(dk, a.kv.kpool + off);
+                    cp_async_16(dk + V, a.kv.vpool + off);
+                } else {
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dk), "r"(0u) : "memory");
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(dk + V), "r"(0u) : "memory");
+                }
             }
         }
         cp_async_commit();
     };
-    const int ntiles = on ? pos / TK + 1 : 0;
-    // old keys: in flight while the kernel ahead finishes (one commit group per tile slot, empty ones included,
-    // so that "all but the newest NBUF - 2 groups" always means "the tile about to be used")
+    const int ngroups = pos >= first_key ? (pos - first_key) / STRIDE + 1 : 0;  // none when the row is off
+    // old keys: in flight while the kernel ahead finishes (one commit group per ring slot, empty ones included,
+    // so that "all but the newest NBUF - 2 groups" always means "the group about to be used")
 #pragma unroll
     for (int p = 0; p < NBUF - 1; ++p) {
-        if (p < ntiles) stage(p * TK, p);
+        if (p < ngroups) stage(p, p);
         else cp_async_commit();
     }
     pdl_wait();
@@ -449,49 +474,50 @@ __global__ void __launch_bounds__(BatchAttnShape<HD, G>::warps * 32, 2)
     float m = -INFINITY, l = 0.f;  // of row qr (a head when qr < G)
     const float inv_sqrt = 1.0f / sqrtf(static_cast<float>(HD));
     trace_mark(trace, 3);
-    for (int it = 0; it < ntiles; ++it) {
-        const int t0 = it * TK, buf = it % NBUF;
-        asm volatile("cp.async.wait_group %0;" ::"n"(NBUF - 2) : "memory");  // this thread's copies of tile `it`
-        __syncthreads();  // everybody's copies of it have landed, and everybody is done with tile it - 1
-        if (it + NBUF - 1 < ntiles) stage((it + NBUF - 1) * TK, (it + NBUF - 1) % NBUF);  // into the buffer tile it - 1 used
+    // ldmatrix rows of this lane: keys (lane & 7) and + 8 for the upper two of a K x4, 8 dims further for the odd ones;
+    // keys (lane & 15) of the values, 8 dims further for the upper half of the lanes
+    const uint32_t k_lane = uint32_t((((lane & 7) + ((lane >> 4) << 3)) * LD + ((lane >> 3) & 1) * 8) * 2);
+    const uint32_t v_lane = uint32_t(((lane & 15) * LD + (lane >> 4) * 8 + P::tile_halves) * 2);
+    for (int g = 0, buf = 0; g < ngroups; ++g, buf = buf + 1 == NBUF ? 0 : buf + 1) {
+        const int t0 = first_key + g * STRIDE;
+        asm volatile("cp.async.wait_group %0;" ::"n"(NBUF - 2) : "memory");  // this lane's copies of group g
+        __syncwarp();  // every lane's copies of it have landed, and every lane is done with group g - 1
+        if (g + NBUF - 1 < ngroups) stage(g + NBUF - 1, buf == 0 ? NBUF - 1 : buf - 1);  // into the buffer group g - 1 used
         else cp_async_commit();
-        __half *kt = tiles + (buf * 2) * P::tile_halves, *vt = tiles + (buf * 2 + 1) * P::tile_halves;
-        if (it == ntiles - 1) {
-            // This step's key and value: rotate k, round both to binary16, into the page and into the tile.
+        const uint32_t tile_u32 = ring_u32 + uint32_t(buf * 2 * P::tile_halves * 2);
+        if (t0 + TK > pos) {
+            // This step's key and value: rotate k, round both to binary16, into the page and into the group.
+            __half *kt = ring + buf * 2 * P::tile_halves, *vt = kt + P::tile_halves;
             const int64_t off = key_offset(pos);
             const float *kh = a.k + size_t(b) * a.kv.kv_dim + size_t(kvh) * HD;
             const float *vh = a.v + size_t(b) * a.kv.kv_dim + size_t(kvh) * HD;
-            for (int idx = tid; idx < HD; idx += P::warps * 32) {
-                const int i = idx % (HD / 2);
-                __half2 h;
-                if (idx < HD / 2) {
-                    const float v0 = kh[2 * i], v1 = kh[2 * i + 1];
-                    h = __halves2half2(__float2half_rn(__fsub_rn(__fmul_rn(v0, cr[i]), __fmul_rn(v1, ci[i]))),
-                                       __float2half_rn(__fadd_rn(__fmul_rn(v0, ci[i]), __fmul_rn(v1, cr[i]))));
-                    *reinterpret_cast<__half2 *>(kt + (pos - t0) * LD + 2 * i) = h;
-                    *reinterpret_cast<__half2 *>(a.kv.kpool + off + 2 * i) = h;
-                } else {
-                    h = __halves2half2(__float2half_rn(vh[2 * i]), __float2half_rn(vh[2 * i + 1]));
-                    *reinterpret_cast<__half2 *>(vt + (pos - t0) * LD + 2 * i) = h;
-                    *reinterpret_cast<__half2 *>(a.kv.vpool + off + 2 * i) = h;
-                }
+            for (int i = lane; i < HD / 2; i += 32) {
+                const float v0 = kh[2 * i], v1 = kh[2 * i + 1];
+                const __half2 hk = __halves2half2(__float2half_rn(__fsub_rn(__fmul_rn(v0, cr[i]), __fmul_rn(v1, ci[i]))),
+                                                  __float2half_rn(__fadd_rn(__fmul_rn(v0, ci[i]), __fmul_rn(v1, cr[i]))));
+                const __half2 hv = __halves2half2(__float2half_rn(vh[2 * i]), __float2half_rn(vh[2 * i + 1]));
+                *reinterpret_cast<__half2 *>(kt + (pos - t0) * LD + 2 * i) = hk;
+                *reinterpret_cast<__half2 *>(vt + (pos - t0) * LD + 2 * i) = hv;
+                *reinterpret_cast<__half2 *>(a.kv.kpool + off + 2 * i) = hk;
+                *reinterpret_cast<__half2 *>(a.kv.vpool + off + 2 * i) = hv;
             }
-            __syncthreads();
+            __syncwarp();
         }
-        const int k0 = 16 * warp;  // this warp's sixteen keys of the tile
-        if (t0 + k0 > pos) continue;
         // S = Q K^T: 16 rows (heads) x 16 keys; separate accumulators for the hi and the lo part of q, so that
         // four chains of MMAs run side by side
         float sh[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, sl[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
             const uint32_t ah[4] = {qhi[k][0], 0u, qhi[k][1], 0u}, al[4] = {qlo[k][0], 0u, qlo[k][1], 0u};
+            uint32_t kf[2][2];  // keys 0-7 and 8-15: dims 0-7 and 8-15 of the step
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(kf[0][0]), "=r"(kf[0][1]), "=r"(kf[1][0]), "=r"(kf[1][1])
+                         : "r"(tile_u32 + k_lane + uint32_t(32 * k))
+                         : "memory");
 #pragma unroll
             for (int nb = 0; nb < 2; ++nb) {
-                const uint32_t b0 = *reinterpret_cast<const uint32_t *>(kt + (k0 + nb * 8 + qr) * LD + 16 * k + 2 * qc);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t *>(kt + (k0 + nb * 8 + qr) * LD + 16 * k + 8 + 2 * qc);
-                mma_16816(sh[nb], ah, b0, b1);
-                mma_16816(sl[nb], al, b0, b1);
+                mma_16816(sh[nb], ah, kf[nb][0], kf[nb][1]);
+                mma_16816(sl[nb], al, kf[nb][0], kf[nb][1]);
             }
         }
         // rows 0..7 are c0 / c1 of each lane: scale, mask the keys after pos, fold into the running soft-max
@@ -501,7 +527,7 @@ __global__ void __launch_bounds__(BatchAttnShape<HD, G>::warps * 32, 2)
         for (int nb = 0; nb < 2; ++nb)
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                sv[nb][c] = (t0 + k0 + nb * 8 + 2 * qc + c <= pos) ? (sh[nb][c] + sl[nb][c]) * inv_sqrt : -INFINITY;
+                sv[nb][c] = (t0 + nb * 8 + 2 * qc + c <= pos) ? (sh[nb][c] + sl[nb][c]) * inv_sqrt : -INFINITY;
                 tmax = fmaxf(tmax, sv[nb][c]);
             }
         tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
@@ -518,23 +544,27 @@ __global__ void __launch_bounds__(BatchAttnShape<HD, G>::warps * 32, 2)
             const __half2 ph = __floats2half2_rn(p0, p1);
             pa[2 * nb] = *reinterpret_cast<const uint32_t *>(&ph);
         }
-        const uint32_t vt_u32 = tiles_u32 + uint32_t((buf * 2 + 1) * P::tile_halves * 2);
 #pragma unroll
-        for (int db = 0; db < DB; ++db) {
-            o[db][0] *= corr;
-            o[db][1] *= corr;
-            uint32_t b0, b1;
-            const uint32_t addr = vt_u32 + uint32_t(((k0 + (lane & 15)) * LD + db * 8) * 2);
-            asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0, %1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(addr));
-            mma_16816(o[db], pa, b0, b1);
+        for (int db = 0; db < DB; db += 2) {
+            uint32_t vf[2][2];
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(vf[0][0]), "=r"(vf[0][1]), "=r"(vf[1][0]), "=r"(vf[1][1])
+                         : "r"(tile_u32 + v_lane + uint32_t(db * 16))
+                         : "memory");
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                o[db + h][0] *= corr;
+                o[db + h][1] *= corr;
+                mma_16816(o[db + h], pa, vf[h][0], vf[h][1]);
+            }
         }
     }
-    // Merge the four warps (each saw a quarter of every tile's keys): per head the maxima, sums and outputs.
+    // Merge the four warps (each saw a quarter of the keys): per head the maxima, sums and outputs.
     trace_mark(trace, 4);
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();  // everybody is done with the tiles: their memory becomes the merge area
+    __syncthreads();  // everybody is done with the rings: their memory becomes the merge area
     if (qr < G) {
         float *mine = merge + (warp * G + qr) * (HD + 2);
 #pragma unroll
