@@ -1,4 +1,4 @@
-// Temperature / top-p sampling on the device: a cluster of eight CTAs per batch row turns the row of
+// Temperature / top-p sampling on the device: a cluster of eight, four or two CTAs per batch row turns the row of
 // logits the vocabulary projection left in device memory into a token id, so that a non-greedy decode
 // step returns 4 bytes per sequence instead of the whole row (513 KB at a 128 256-token vocabulary).
 //
@@ -19,8 +19,8 @@
 // together hold less than 1 - topp, so the running sum passes topp before it reaches them - and is not needed.
 // Nothing is sorted: "the element where the running sum, largest first, crosses t" is found by descending the
 // binary32 bit pattern of e (non-negative floats order like their bits) 11 + 11 + 9 bits at a time: each CTA
-// builds a histogram (count and sum per bucket) of its eighth of the row over the elements that match the
-// prefix found so far, the cluster's first CTA adds the eight histograms through distributed shared memory,
+// builds a histogram (count and sum per bucket) of its share of the row over the elements that match the
+// prefix found so far, the cluster's first CTA adds the histograms through distributed shared memory,
 // scans from the top to the bucket where the sum crosses, and hands the result back. Sums are exact integers
 // (e x 2^40 in 64 bits), so the result does not depend on the order of the additions: the same row and the
 // same u give the same token on every run, and ties go in index order. Against the reference's sequential
@@ -34,7 +34,7 @@ namespace jl {
 
 namespace {
 
-constexpr int kCluster = 8;
+constexpr int kMaxCluster = 8;
 constexpr int kSampleThreads = 1024;
 constexpr int kSampleWarps = kSampleThreads / 32;
 constexpr int kBuckets = 2048;
@@ -54,7 +54,7 @@ struct Pick {  // what a scan of a merged histogram found
 
 struct SampleSmem {
     // this CTA's histogram of the current level: the sum of a bucket in three 32-bit limbs of 14 bits each
-    // (a slice has at most 2^16 elements of 41 bits), because shared memory adds 32-bit words natively while a
+    // (a slice has at most 2^18 elements of 41 bits), because shared memory adds 32-bit words natively while a
     // 64-bit addition there is a compare-and-swap loop that many warps on a few buckets keep retrying
     unsigned hlimb[3][kBuckets];
     unsigned hcnt[kBuckets];
@@ -64,9 +64,9 @@ struct SampleSmem {
     unsigned wcnt[kSampleWarps];
     float wred[kSampleWarps];
     // one slot per CTA of the cluster, written by its owner into every CTA's copy
-    float cmax[kCluster];
-    unsigned long long csum[kCluster];
-    unsigned long long ccnt[kCluster];
+    float cmax[kMaxCluster];
+    unsigned long long csum[kMaxCluster];
+    unsigned long long ccnt[kMaxCluster];
     Pick pick;  // written by the first CTA into every CTA's copy
     float fval;
     int ival;
@@ -176,9 +176,10 @@ __device__ void hist_pass(const float *e, const float (&kept)[kKeep], int lo, in
 }
 
 // First CTA only: scans a histogram (buckets from the top) for the bucket where `above + running sum` first
-// exceeds `target`, and writes the result into every CTA's copy of `pick`. `merge`: add the eight CTAs'
+// exceeds `target`, and writes the result into every CTA's copy of `pick`. `merge`: add the C CTAs'
 // histograms on the fly (and keep the sums in g1 when `keep`); otherwise scan g1.
 // `frac` >= 0 (first level only): the target is that fraction of the row's total mass, which this scan also finds.
+template <int C>
 __device__ void scan_and_publish(SampleSmem &sm, int bits, bool merge, bool keep, unsigned long long above,
                                  unsigned long long target, double frac) {
     const int tid = threadIdx.x, lane = tid & 31;
@@ -190,16 +191,16 @@ __device__ void scan_and_publish(SampleSmem &sm, int bits, bool merge, bool keep
         const int b = nb - 1 - (tid * per + k);
         if (b < 0) continue;
         if (merge) {
-            unsigned t0[kCluster], t1[kCluster], t2[kCluster], tc[kCluster];
+            unsigned t0[C], t1[C], t2[C], tc[C];
 #pragma unroll
-            for (uint32_t r = 0; r < kCluster; ++r) {
+            for (uint32_t r = 0; r < C; ++r) {
                 t0[r] = ld_remote_u32(&sm.hlimb[0][b], r);
                 t1[r] = ld_remote_u32(&sm.hlimb[1][b], r);
                 t2[r] = ld_remote_u32(&sm.hlimb[2][b], r);
                 tc[r] = ld_remote_u32(&sm.hcnt[b], r);
             }
 #pragma unroll
-            for (uint32_t r = 0; r < kCluster; ++r) {
+            for (uint32_t r = 0; r < C; ++r) {
                 s[k] += static_cast<unsigned long long>(t0[r]) + (static_cast<unsigned long long>(t1[r]) << 14) +
                         (static_cast<unsigned long long>(t2[r]) << 28);
                 c[k] += tc[r];
@@ -246,7 +247,7 @@ __device__ void scan_and_publish(SampleSmem &sm, int bits, bool merge, bool keep
     const int owner = sm.ival;
     if (owner < 0 && tid == 0) p.above = total;  // never exceeds the target: report the whole mass
     if (tid == (owner < 0 ? 0 : owner)) {
-        for (uint32_t r = 0; r < kCluster; ++r) {
+        for (uint32_t r = 0; r < C; ++r) {
             st_remote_u64(&sm.pick.above, r, p.above);
             st_remote_u64(&sm.pick.bsum, r, p.bsum);
             st_remote_u32(&sm.pick.bcnt, r, p.bcnt);
@@ -269,6 +270,7 @@ struct Crossing {
 // first CTA's g1; otherwise this CTA's first-level histogram has just been built in hsum / hcnt. Every CTA
 // of the cluster calls this with the same arguments.
 // `frac` >= 0: the target is that fraction of the row's mass (known only after the first level's scan).
+template <int C>
 __device__ Crossing find_crossing(const float *e, const float (&kept)[kKeep], int lo, int hi, unsigned long long target, double frac,
                                   bool first_level_ready, uint32_t crank, SampleSmem &sm) {
     Crossing c = {false, 0u, 0u, 0ull, 0ull};
@@ -281,7 +283,7 @@ __device__ Crossing find_crossing(const float *e, const float (&kept)[kKeep], in
         const bool reuse = lv == 0 && first_level_ready;
         if (lv > 0) hist_pass(e, kept, lo, hi, prefix, known, level_bits[lv], sm);
         if (!reuse) cluster_sync();  // every CTA's histogram of this level is complete
-        if (crank == 0) scan_and_publish(sm, level_bits[lv], !reuse, lv == 0, above, target, lv == 0 ? frac : -1.0);
+        if (crank == 0) scan_and_publish<C>(sm, level_bits[lv], !reuse, lv == 0, above, target, lv == 0 ? frac : -1.0);
         cluster_sync();  // the result is in every CTA's `pick`; the histograms may be cleared again
         pk = sm.pick;
         if (lv == 0) {
@@ -309,14 +311,16 @@ __device__ Crossing find_crossing(const float *e, const float (&kept)[kKeep], in
 }
 
 // One value per CTA (slices are in index order) into every CTA's `slots`; returns what comes before this CTA's.
+template <int C>
 __device__ unsigned long long cluster_exclusive(unsigned long long mine, unsigned long long *slots, uint32_t crank) {
-    if (threadIdx.x < kCluster) st_remote_u64(&slots[crank], threadIdx.x, mine);
+    if (threadIdx.x < C) st_remote_u64(&slots[crank], threadIdx.x, mine);
     cluster_sync();
     unsigned long long before = 0ull;
     for (uint32_t r = 0; r < crank; ++r) before += slots[r];
     return before;
 }
 
+template <int C>
 __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logits, int vocab, const uint8_t *active,
                                                                      float temperature, float topp, const float *uniforms,
                                                                      const int32_t *greedy, int32_t *out) {
@@ -330,7 +334,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
     }
     float *e = logits + size_t(row) * vocab;
     const int n = vocab;
-    const int per_cta = ((n + kCluster - 1) / kCluster + 3) & ~3;
+    const int per_cta = ((n + C - 1) / C + 3) & ~3;
     const int lo = min(n, int(crank) * per_cta), hi = min(n, lo + per_cta);
     // scores / temperature and their maximum over the row: the step's arg-max kernel has already found where
     // the maximum sits (greedy may alias out: it is read here, out is written at the very end)
@@ -342,11 +346,11 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
         mx = -INFINITY;
         for (int i = lo + tid; i < hi; i += kSampleThreads) mx = fmaxf(mx, __fdiv_rn(e[i], temperature));
         mx = block_max(mx, sm);
-        if (tid < kCluster)
+        if (tid < C)
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote_addr(&sm.cmax[crank], uint32_t(tid))), "f"(mx) : "memory");
         cluster_sync();
         mx = sm.cmax[0];
-        for (int r = 1; r < kCluster; ++r) mx = fmaxf(mx, sm.cmax[r]);
+        for (int r = 1; r < C; ++r) mx = fmaxf(mx, sm.cmax[r]);
     }
     // e = exp(score - max) in place, and (for the nucleus sampler) this CTA's first-level histogram of it in the same pass
     const bool nucleus_mode = topp > 0.0f && topp < 1.0f;
@@ -407,9 +411,9 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
         __syncthreads();
         unsigned long long cta_total = 0ull;
         for (int w = 0; w < kSampleWarps; ++w) cta_total += sm.wsum[w];
-        unsigned long long before = cluster_exclusive(cta_total, sm.csum, crank);
+        unsigned long long before = cluster_exclusive<C>(cta_total, sm.csum, crank);
         unsigned long long total = 0ull;
-        for (int r = 0; r < kCluster; ++r) total += sm.csum[r];
+        for (int r = 0; r < C; ++r) total += sm.csum[r];
         const unsigned long long target =
             static_cast<unsigned long long>(static_cast<double>(u) * static_cast<double>(total));  // cdf > u  <=>  running e > u * sum
         for (int w = 0; w < (tid >> 5); ++w) before += sm.wsum[w];
@@ -424,20 +428,20 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
                 }
             }
         }
-        if (crank == kCluster - 1 && tid == kSampleThreads - 1 && target >= total) out[row] = n - 1;  // CategoricalSampler.java:24
+        if (crank == C - 1 && tid == kSampleThreads - 1 && target >= total) out[row] = n - 1;  // CategoricalSampler.java:24
         cluster_sync();  // nobody leaves while its shared memory may still be written
         return;
     }
     // ToppSampler. Stage 1: where the running sum, largest first, exceeds topp * sum (the first scan also yields the
     // sum and leaves the merged first-level histogram with the first CTA).
-    const Crossing nucleus = find_crossing(e, kept, lo, hi, 0ull, static_cast<double>(topp), false, crank, sm);
+    const Crossing nucleus = find_crossing<C>(e, kept, lo, hi, 0ull, static_cast<double>(topp), false, crank, sm);
     const unsigned long long total = nucleus.total;
     // Stage 2: r = u * (that running sum as a probability), ToppSampler.java:92, and where the running sum exceeds it.
     const float mass_p = static_cast<float>(static_cast<double>(nucleus.mass) / static_cast<double>(total));
     const float r = __fmul_rn(u, mass_p);
     unsigned long long t2 = static_cast<unsigned long long>(static_cast<double>(r) * static_cast<double>(total));
     if (nucleus.mass > 0ull && t2 >= nucleus.mass) t2 = nucleus.mass - 1ull;  // u * mass rounded up to the mass: its last element
-    const Crossing pick = find_crossing(e, kept, lo, hi, t2, -1.0, true, crank, sm);
+    const Crossing pick = find_crossing<C>(e, kept, lo, hi, t2, -1.0, true, crank, sm);
     const Crossing use = pick.found ? pick : nucleus;
     if (use.found) {
         // The rank-th element (index order) with exactly this key.
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
         __syncthreads();
         unsigned cta_total = 0u;
         for (int w = 0; w < kSampleWarps; ++w) cta_total += sm.wcnt[w];
-        unsigned before = unsigned(cluster_exclusive(cta_total, sm.ccnt, crank));
+        unsigned before = unsigned(cluster_exclusive<C>(cta_total, sm.ccnt, crank));
         for (int w = 0; w < (tid >> 5); ++w) before += sm.wcnt[w];
         before += incl - mine;
         if (before < use.rank && use.rank <= before + mine) {
@@ -471,29 +475,52 @@ __global__ void __launch_bounds__(kSampleThreads) sample_rows_kernel(float *logi
     cluster_sync();  // nobody leaves while its shared memory may still be read or written
 }
 
-}  // namespace
-
-cudaError_t sample_rows_configure() {
-    return cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SampleSmem)));
+template <int C>
+cudaError_t sample_rows_configure_c() {
+    return cudaFuncSetAttribute(sample_rows_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(sizeof(SampleSmem)));
 }
 
-cudaError_t sample_rows_launch(float *logits, int vocab, int width, const uint8_t *active, float temperature, float topp,
-                               const float *uniforms, const int32_t *greedy, int32_t *out, cudaStream_t stream) {
-    if (logits == nullptr || uniforms == nullptr || out == nullptr || vocab < 2 || width < 1 || !(temperature > 0.0f))
-        return cudaErrorInvalidValue;
+template <int C>
+cudaError_t sample_rows_launch_c(float *logits, int vocab, int width, const uint8_t *active, float temperature, float topp,
+                                 const float *uniforms, const int32_t *greedy, int32_t *out, cudaStream_t stream) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kCluster, unsigned(width));
+    cfg.gridDim = dim3(C, unsigned(width));
     cfg.blockDim = dim3(kSampleThreads);
     cfg.dynamicSmemBytes = sizeof(SampleSmem);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kCluster;
+    attr[0].val.clusterDim.x = C;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, sample_rows_kernel, logits, vocab, active, temperature, topp, uniforms, greedy, out);
+    return cudaLaunchKernelEx(&cfg, sample_rows_kernel<C>, logits, vocab, active, temperature, topp, uniforms, greedy, out);
+}
+
+}  // namespace
+
+cudaError_t sample_rows_configure() {
+    cudaError_t e = sample_rows_configure_c<8>();
+    if (e == cudaSuccess) e = sample_rows_configure_c<4>();
+    if (e == cudaSuccess) e = sample_rows_configure_c<2>();
+    return e;
+}
+
+// How many CTAs share a row. A CTA of 1024 threads with 64 registers fills an SM, and a row costs mostly the
+// descent's fixed part (barriers of the cluster, the merge of the histograms over distributed shared memory), which a
+// wider cluster does not shorten: so the widest cluster with which the rows still make one wave. Of clusters of
+// eight about 16 fit on the chip at once (a cluster stays within one GPC), of four 32. At 128 256 tokens, top-p 0.95: one
+// row takes 80 us with 8 CTAs, 100 with 4, 127 with 2; 64 rows take 391, 207, 137 (with one CTA each 227).
+// A slice holds at most 2^18 elements (the histogram's limbs), which only vocabularies past half a million reach.
+cudaError_t sample_rows_launch(float *logits, int vocab, int width, const uint8_t *active, float temperature, float topp,
+                               const float *uniforms, const int32_t *greedy, int32_t *out, cudaStream_t stream) {
+    if (logits == nullptr || uniforms == nullptr || out == nullptr || vocab < 2 || width < 1 || !(temperature > 0.0f))
+        return cudaErrorInvalidValue;
+    const auto launch = width > 32 && vocab <= (2 << 18)   ? sample_rows_launch_c<2>
+                        : width > 16 && vocab <= (4 << 18) ? sample_rows_launch_c<4>
+                                                           : sample_rows_launch_c<8>;
+    return launch(logits, vocab, width, active, temperature, topp, uniforms, greedy, out, stream);
 }
 
 }  // namespace jl

@@ -10,7 +10,7 @@ namespace jl {
 // logits[width][vocab] for temperature > 0, nucleus threshold topp (outside (0,1): plain categorical sampling)
 // and the uniform random number uniforms[r] in [0,1); -1 for rows whose active flag is 0. The rows are
 // `greedy` (nullable; may alias out): the index of each row's maximum, which spares a pass. The rows are
-// overwritten with exp(score - max), as the reference overwrites its logits. A cluster of eight CTAs per row.
+// overwritten with exp(score - max), as the reference overwrites its logits. A cluster of eight, four or two CTAs per row.
 // Sets the kernel's shared-memory attribute (call once per device, outside stream capture).
 cudaError_t sample_rows_configure();
 cudaError_t sample_rows_launch(float *logits, int vocab, int width, const uint8_t *active, float temperature, float topp,
