@@ -141,7 +141,8 @@ __global__ void tp_pick_best_kernel(const float *all, int ranks, int n, const ui
 // ---- row-wise operators for the matrix-matrix path ---------------------------------------------
 // One CTA per row. The row is read once, as float4 batches held in registers (all loads issued
 // before the first use: one L2 round trip, not one per element), and the same registers feed the
-// output pass. Optionally also writes the row as binary16 hi / lo parts (x = hi + lo), the
+// output pass. The norm's weights, which no kernel writes, are in flight while the kernel ahead still runs: loaded after
+// the sum they cost a second round trip, to memory (65 such launches in a step of 32 rows: 4192 -> 4110 us). Optionally also writes the row as binary16 hi / lo parts (x = hi + lo), the
 // activation format of the tensor-core path.
 constexpr int kNormThreads = 256;
 constexpr int kNormBatch = 8;  // float4 per thread per batch: rows up to 8192 in one batch
@@ -152,13 +153,18 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float 
     const int trace = trace_begin(kTraceRows);
     trace_word(trace, 7, 1);
     pdl_launch_dependents();
-    pdl_wait();
-    if (active != nullptr && active[row] == 0) return;
     __shared__ float part[9];
     const int n4 = dim / 4;
     const float4 *xr = reinterpret_cast<const float4 *>(x + size_t(row) * dim);
     const float4 *w4 = reinterpret_cast<const float4 *>(w);
-    float4 v[kNormBatch];
+    float4 v[kNormBatch], g[kNormBatch];
+#pragma unroll
+    for (int k = 0; k < kNormBatch; ++k) {
+        const int i = k * kNormThreads + threadIdx.x;
+        g[k] = i < n4 ? w4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    pdl_wait();
+    if (active != nullptr && active[row] == 0) return;
 #pragma unroll
     for (int k = 0; k < kNormBatch; ++k) {
         const int i = k * kNormThreads + threadIdx.x;
@@ -186,8 +192,7 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float 
     float4 *o4 = reinterpret_cast<float4 *>(out + size_t(row) * dim);
     uint2 *hr = hi != nullptr ? hi + size_t(row) * n4 : nullptr;
     uint2 *lr = lo != nullptr ? lo + size_t(row) * n4 : nullptr;
-    auto emit = [&](int i, float4 u) {
-        const float4 g = w4[i];
+    auto emit = [&](int i, float4 u, float4 g) {
         float4 r;
         r.x = __fmul_rn(g.x, __fmul_rn(ss, u.x));
         r.y = __fmul_rn(g.y, __fmul_rn(ss, u.y));
@@ -199,9 +204,9 @@ __global__ void __launch_bounds__(kNormThreads) rmsnorm_rows_kernel(const float 
 #pragma unroll
     for (int k = 0; k < kNormBatch; ++k) {
         const int i = k * kNormThreads + threadIdx.x;
-        if (i < n4) emit(i, v[k]);
+        if (i < n4) emit(i, v[k], g[k]);
     }
-    for (int i = kNormBatch * kNormThreads + threadIdx.x; i < n4; i += kNormThreads) emit(i, xr[i]);
+    for (int i = kNormBatch * kNormThreads + threadIdx.x; i < n4; i += kNormThreads) emit(i, xr[i], w4[i]);
 }
 
 // Four elements per thread per step (row lengths are multiples of 256, so float4 never straddles).
