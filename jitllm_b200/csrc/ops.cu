@@ -142,8 +142,9 @@ __global__ void tp_pick_best_kernel(const float *all, int ranks, int n, const ui
 // One CTA per row. The row is read once, as float4 batches held in registers (all loads issued
 // before the first use: one L2 round trip, not one per element), and the same registers feed the
 // output pass. The norm's weights, which no kernel writes, are in flight while the kernel ahead still runs: loaded after
-// the sum they cost a second round trip, to memory (65 such launches in a step of 32 rows: 4192 -> 4110 us). Optionally also writes the row as binary16 hi / lo parts (x = hi + lo), the
-// activation format of the tensor-core path.
+// the sum they cost a second round trip, to memory (65 such launches in a step of 32 rows: 4192 -> 4110 us).
+// Optionally also writes the row as binary16 hi / lo parts (x = hi + lo), the activation format of the
+// tensor-core path.
 constexpr int kNormThreads = 256;
 constexpr int kNormBatch = 8;  // float4 per thread per batch: rows up to 8192 in one batch
 
@@ -253,8 +254,8 @@ __global__ void kv_append_kernel(const float *k, const float *v, const float *ro
 // The first index of each row's maximum, one CTA of 1024 threads per row. A row of 128 256 logits is 513 KB and sits in
 // L2 (the projection just wrote it), so the kernel is bound by the loads a CTA keeps in flight: with 4-byte loads
 // issued between the comparisons, 126 to a thread, it was a chain of round trips; eight 16-byte loads in flight leave
-// four of them (a step of 32 rows 4540 -> 4519 us). Rows that do not start on 16 bytes (a vocabulary that is no multiple of 4) take eight 4-byte
-// loads instead.
+// four of them (a step of 32 rows 4540 -> 4519 us). Rows that do not start on 16 bytes (a vocabulary that is no
+// multiple of 4) take eight 4-byte loads instead.
 constexpr int kArgmaxLoads = 8;
 
 __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *logits, int vocab, const uint8_t *active,
