@@ -6,12 +6,16 @@
 // (tensor/standard/ArrayHalfFloatTensor.java:33-40).
 //
 // One CTA of eight warps = (range of keys, KV head, row). The G query heads that share the KV head are rows of one MMA
-// tile: a query, and a probability, is the exact sum of three binary16 parts, which are three rows each (3 G <= 12 of the 16
-// rows; G = 8 takes two tiles), so q.k and p.v keep their 32 bits while keys and values are binary16 as stored. Tiles of 64
-// keys come through a double buffer by cp.async; warp w multiplies sixteen of a tile's keys and half of the output dimensions.
-// A launch is latency: 64 keys per CTA as long as there are CTAs, then longer ranges. The last CTA of a (row, KV head) to
-// finish folds the ranges' results; the arrival is one atomic. The kernel before this one took scalar products (8 keys per
-// warp in 1.2 us) and folded sixteen warps and a cluster of eight CTAs (2.5 us).
+// tile: a query, scaled by a power of two from its head's largest element, and a probability are each the sum of three
+// binary16 parts, which are three rows each (3 G <= 12 of the 16 rows; G = 8 takes two tiles), so q.k and p.v keep their 32
+// bits (split3 says down to which size) while keys and values are binary16 as stored. Tiles of 64 keys come through a double
+// buffer by cp.async; warp w multiplies sixteen of a tile's keys and half of the output dimensions. A launch is latency: 64
+// keys per CTA as long as there are CTAs, then longer ranges. The last CTA of a (row, KV head) to finish folds the ranges'
+// results; the arrival is one atomic.
+// Error against a 64-bit softmax over the same query, keys and values (2-norm; geometric mean over 20 models, head sizes 64
+// and 128, groups of 2, 4 and 8, scores of standard deviation 0.2 to 8, 1 to 3000 keys): 1.47e-7; scalar binary32 sums in the
+// split of the keys that a kernel of scalar products would take 1.50e-7. It does not depend on the size of the queries
+// (2^-12 to 2^15 times the usual one: 2.4e-7 to 2.7e-7 where it is 2.5e-7), nor on how the heads of a group compare.
 #include "ops.cuh"
 
 #include <cuda_bf16.h>
@@ -42,27 +46,48 @@ __device__ __forceinline__ void ldmatrix4_trans(uint32_t (&r)[4], uint32_t addr)
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) { asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory"); }
-// x as the sum of three binary16 values of eight significant bits each: all 24 of it. (Not of eleven: the tensor core cuts its
-// sums of sixteen products off at some 2^-24 of the largest, and a part's products with binary16 keys would reach below that.
-// Eight bits leave the first part's sums whole, and what is cut off the other two is 2^-8 and 2^-16 of it.)
+// x, at most 2^15 in magnitude, as the sum of three binary16 values of eight significant bits each: all 24 bits from 1/2 up, and
+// below that all of them down to 2^-24, where binary16 ends (what is lost is at most 2^-25). The callers scale what they split by
+// a power of two so that its largest lies between 2^14 and 2^15: every value down to 2^-15 of the largest is whole, and what the
+// smaller ones lose is at most 2^-39 of the largest. (Parts of eight bits, not of eleven: the tensor core cuts its sums of sixteen
+// products off at some 2^-24 of the largest, and a part's products with binary16 keys would reach below that. Eight bits leave
+// the first part's sums whole, and what is cut off the other two is 2^-8 and 2^-16 of it.)
 __device__ __forceinline__ void split3(float x, __half (&h)[3]) {
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-        const float part = __bfloat162float(__float2bfloat16_rn(x));
-        h[p] = __float2half_rn(part);
-        x -= part;
+        h[p] = __float2half_rn(__bfloat162float(__float2bfloat16_rn(x)));
+        x -= __half2float(h[p]);  // exact; with what binary16 dropped of the part
     }
     h[2] = __float2half_rn(x);
+}
+// The power of two that takes a largest magnitude (its bits, finite) to between 2^14 and 2^15, as bits; 2^100 for those below 2^-86,
+// whose scores are all but equal.
+__device__ __forceinline__ unsigned query_scale(unsigned most) { return min(268u - (most >> 23), 227u) << 23; }
+// The sum of 2^n values in n roundings.
+template <int N>
+__device__ __forceinline__ float sum_pairs(const float (&x)[N]) {
+    float s[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) s[i] = x[i];
+#pragma unroll
+    for (int w = 1; w < N; w *= 2)
+#pragma unroll
+        for (int i = 0; i < N; i += 2 * w) s[i] += s[i + w];
+    return s[0];
 }
 
 template <int HD, int G>
 struct SplitAttn {
     static constexpr int LD = HD + 8;          // halves per row: no bank conflicts
     static constexpr int QT = G == 8 ? 2 : 1;  // sixteen-row tiles that hold three parts of G heads
+    // The row of a head's part. The sum over the parts starts with rows r and r + 8: the two small parts meet first, so that the
+    // large one is rounded once.
+    static __host__ __device__ constexpr int row(int part, int g) { return part < 2 ? part * G + g : G == 8 ? 16 + g : 8 + G + g; }
     struct Smem {
         alignas(16) __half q[QT * 16][LD];
         int pages[kPages];
         float w[kGroups][G];  // merge weights
+        unsigned q_most[G * HD / 64];  // the largest finite magnitude of every 64 elements of the rotated queries, as bits
         float inv[G], sum[G], top[G];
         int is_last;
         union {
@@ -146,7 +171,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
     // Queries rotated, and the new key and value: rotated, rounded to binary16 as the append does.
     float qx[kRounds] = {}, qy[kRounds] = {};
     uint32_t fresh[kRounds] = {};
-    bool large = false;
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
         const int idx = tid + r * kThreads, i = idx % (HD / 2);
@@ -154,7 +178,10 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
             const float2 x = __ldcg(reinterpret_cast<const float2 *>(a.q + size_t(b) * a.dim + size_t(kvh * G + idx / (HD / 2)) * HD) + i);
             qx[r] = __fsub_rn(__fmul_rn(x.x, cr[r]), __fmul_rn(x.y, ci[r]));
             qy[r] = __fadd_rn(__fmul_rn(x.x, ci[r]), __fmul_rn(x.y, cr[r]));
-            large = large || fmaxf(fabsf(qx[r]), fabsf(qy[r])) > 32768.0f;
+            // the lanes of a warp have 64 elements of one head
+            const unsigned ax = __float_as_uint(fabsf(qx[r])), ay = __float_as_uint(fabsf(qy[r])), inf = 0x7f800000u;
+            const unsigned most = __reduce_max_sync(0xffffffffu, max(ax < inf ? ax : 0u, ay < inf ? ay : 0u));
+            if (lane == 0) sm.q_most[idx / 32] = most;
         } else if (owns_new && idx < kPairs) {
             const bool is_k = idx < (G + 1) * (HD / 2);
             const float2 x = __ldcg(reinterpret_cast<const float2 *>((is_k ? a.k : a.v) + size_t(b) * kv_dim + size_t(kvh) * HD) + i);
@@ -166,35 +193,28 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
             fresh[r] = *reinterpret_cast<const uint32_t *>(&h);
         }
     }
-    // Queries beyond the range of binary16 are scaled by a power of two (the same for all ranges: they see the same queries).
-    float q_scale = 1.0f;
-    if (__syncthreads_or(large)) {
-        if (tid == 0) sm.is_last = 0;
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-            const float most = fmaxf(fabsf(qx[r]), fabsf(qy[r]));
-            if (most < INFINITY) atomicMax(&sm.is_last, __float_as_int(most));
-        }
-        __syncthreads();
-        q_scale = exp2f(static_cast<float>(14 - ((sm.is_last >> 23) - 127)));
-    }
+    // Every head's query is scaled by a power of two from its own largest element (the same for all ranges: they see the same
+    // queries), so that the split keeps its bits whatever its magnitude and whatever its neighbours'.
+    __syncthreads();
+    auto scale_of = [&](int g) { return query_scale(HD == 64 ? sm.q_most[g] : max(sm.q_most[2 * g], sm.q_most[2 * g + 1])); };
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
         const int idx = tid + r * kThreads, i = idx % (HD / 2);
         if (idx < G * (HD / 2)) {
             const int g = idx / (HD / 2);
             __half p0[3], p1[3];
-            split3(qx[r] * q_scale, p0);
-            split3(qy[r] * q_scale, p1);
+            const float scale = __uint_as_float(scale_of(g));
+            split3(qx[r] * scale, p0);
+            split3(qy[r] * scale, p1);
 #pragma unroll
-            for (int p = 0; p < 3; ++p) *reinterpret_cast<__half2 *>(&sm.q[p * G + g][2 * i]) = __halves2half2(p0[p], p1[p]);
+            for (int p = 0; p < 3; ++p) *reinterpret_cast<__half2 *>(&sm.q[A::row(p, g)][2 * i]) = __halves2half2(p0[p], p1[p]);
         }
     }
     trace_mark(trace, 3);
-    const float inv_sqrt = 1.0f / sqrtf(static_cast<float>(HD)), unscale = 1.0f / q_scale;
     const int gl = lane >> 2, t = lane & 3, kg = warp & (kGroups - 1), half = warp / kGroups;
-    constexpr float kUp = 4096.0f;  // probabilities are split as multiples of 2^-12: the small ones' parts stay normal
+    // 1 / sqrt(head size), and the scale of this lane's head taken back (exactly)
+    const float to_score = (1.0f / sqrtf(static_cast<float>(HD))) * __uint_as_float((254u << 23) - scale_of(gl % G));
+    constexpr float kUp = 32768.0f;  // probabilities, at most 1, are split as multiples of 2^-15
     float m = -INFINITY, l = 0.f, o[DB][4];
 #pragma unroll
     for (int d = 0; d < DB; ++d) o[d][0] = o[d][1] = o[d][2] = o[d][3] = 0.f;
@@ -272,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int key = t0 + key0 + (c >> 1) * 8 + 2 * t + (c & 1);
-            s[c] = key < end ? s[c] * unscale * inv_sqrt : -INFINITY;
+            s[c] = key < end ? s[c] * to_score : -INFINITY;
             top = fmaxf(top, s[c]);
         }
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
@@ -281,16 +301,15 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
         // every score of the group may be -inf (an infinite query or key): no weight, as the reference's exp(-inf - max)
         const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
         m = mn;
-        l *= corr;
         uint32_t pf[QT][4];
         __half part[4][3];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const float p = mn == -INFINITY ? 0.f : expf(s[c] - mn);
-            l += p;
-            split3(p * kUp, part[c]);
+            s[c] = mn == -INFINITY ? 0.f : expf(s[c] - mn);
+            split3(s[c] * kUp, part[c]);
         }
-        // rows gl and gl + 8 of the probability tile(s): part row / G of head row % G
+        l = fmaf(l, corr, (s[0] + s[1]) + (s[2] + s[3]));
+        // rows gl and gl + 8 of the probability tile(s), laid out as the queries'
 #pragma unroll
         for (int f = 0; f < 2; ++f) {
             uint32_t w[3];
@@ -306,8 +325,8 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
                 pf[QT - 1][2 * f] = w[2];
                 pf[QT - 1][2 * f + 1] = 0u;
             } else {
-                pf[0][2 * f] = which == 0 ? w[0] : which == 1 ? w[1] : which == 2 ? w[2] : 0u;
-                pf[0][2 * f + 1] = G == 4 && which == 0 ? w[2] : 0u;
+                pf[0][2 * f] = which == 0 ? w[0] : which == 1 ? w[1] : 0u;
+                pf[0][2 * f + 1] = which == 1 ? w[2] : 0u;
             }
         }
         const uint32_t va = v0 + uint32_t((buf * kTile + key0 + (lane & 15)) * LD + half * (HD / 2) + (lane >> 4) * 8) * 2;
@@ -367,9 +386,10 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
     float *parts = a.partial + (size_t(b) * a.kv_heads + kvh) * a.nsplit * (G * ROW);  // [range][head][HD + 2]
     for (int idx = tid; idx < G * HD; idx += kThreads) {
         const int g = idx / HD, d = idx - g * HD;
-        float val = 0.f;
+        float part[kGroups];
 #pragma unroll
-        for (int w = 0; w < kGroups; ++w) val += sm.merge[w][g][d] * sm.w[w][g];
+        for (int w = 0; w < kGroups; ++w) part[w] = sm.merge[w][g][d] * sm.w[w][g];
+        const float val = sum_pairs(part);
         if (nsplit == 1) {
             attn_store(a, size_t(b), (kvh * G + g) * HD + d, val / sm.sum[g]);
         } else {
@@ -427,17 +447,18 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
         const int idx = tid + r * kThreads;
         if (idx >= G * HD) break;
         const int g = idx / HD, d = idx - g * HD;
-        float val = 0.f;
+        float early[kEarly];
 #pragma unroll
-        for (int s = 0; s < kEarly; ++s)
-            if (s < nsplit) val += mine[r][s] * sm.fold[s * G + g];
+        for (int s = 0; s < kEarly; ++s) early[s] = s < nsplit ? mine[r][s] * sm.fold[s * G + g] : 0.f;
+        float val = sum_pairs(early);
         for (int s0 = kEarly; s0 < nsplit; s0 += 8) {
             float more[8];
 #pragma unroll
             for (int s = 0; s < 8; ++s) more[s] = s0 + s < nsplit ? __ldcg(parts + (size_t(s0 + s) * G + g) * ROW + d) : 0.f;
 #pragma unroll
             for (int s = 0; s < 8; ++s)
-                if (s0 + s < nsplit) val += more[s] * sm.fold[(s0 + s) * G + g];
+                if (s0 + s < nsplit) more[s] *= sm.fold[(s0 + s) * G + g];
+            val += sum_pairs(more);
         }
         attn_store(a, size_t(b), (kvh * G + g) * HD + d, val * sm.inv[g]);
     }

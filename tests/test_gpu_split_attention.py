@@ -1,12 +1,12 @@
 """Decode attention with the keys split over CTAs, by itself: the attention output of a one-layer model's step against a 64-bit
 softmax over the query, keys and values that the device itself used (the projections and pages are read back), at the depths
 where the split changes: one key, around one tile of 64, where a second range, a third and the last of twenty begin, and
-where ranges grow beyond a tile; every head size and group."""
+where ranges grow beyond a tile; every head size and group; queries of every magnitude."""
 import numpy as np
 import pytest
 
 import jitllm_b200 as jl
-from jitllm_b200 import GGMLType
+from jitllm_b200 import GGMLType, TensorRole
 from tests.util import rel_l2
 
 pytestmark = pytest.mark.gpu
@@ -15,11 +15,14 @@ pytestmark = pytest.mark.gpu
 BAR = 1e-5
 
 
-def attention_errors(dev, rope, heads, kv_heads, head, page, depths, width=1, std=0.05, seed=3):
-    """rel-L2 of the attention outputs of one step at every depth (keys in the pages before it)."""
+def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, std=0.05, seed=3, edit=None):
+    """(output, 64-bit output, rotated query), [head][dimension] each, of one step at every depth (keys in the pages before it).
+    `edit` changes the tensors."""
     cfg = jl.Configuration(dim=heads * head, hiddenDim=512, numberOfLayers=1, numberOfHeads=heads, numberOfKeyValueHeads=kv_heads,
                            vocabularySize=512, contextLength=max(depths) + 16)
     tensors = jl.synth_model_tensors(cfg, GGMLType.Q8_0, seed=seed, std=std)
+    if edit is not None:
+        edit(cfg, tensors)
     cr, ci = rope(cfg)
     model = jl.load_model(dev, cfg, tensors, cr, ci, maxBatch=width)
     bps = (cfg.contextLength + page - 1) // page
@@ -42,19 +45,43 @@ def attention_errors(dev, rope, heads, kv_heads, head, page, depths, width=1, st
             q = q.reshape(heads, head).astype(np.float64)
             k, v = (np.stack([kv.readRow(w, b, 0, i).view(np.float16) for i in range(p + 1)]).astype(np.float64).reshape(p + 1, kv_heads, head)
                     for w in ("k", "v"))
-            got = model.debugRead("xb", b)
+            got = model.debugRead("xb", b).reshape(heads, head)
             want = np.empty((heads, head))
             for h in range(heads):
                 s = k[:, h * kv_heads // heads] @ q[h] / np.sqrt(head)
                 w = np.exp(s - s.max())
                 want[h] = (w / w.sum()) @ v[:, h * kv_heads // heads]
-            out.append(rel_l2(got, want.reshape(-1)))
+            out.append((got, want, q))
     kv.close()
     return out
 
 
+def attention_errors(*args, **kwargs):
+    """rel-L2 of the attention outputs of one step at every depth."""
+    return [rel_l2(got.reshape(-1), want.reshape(-1)) for got, want, _ in attention_outputs(*args, **kwargs)]
+
+
 def _rope(cfg):
     return jl.precomputeFreqsCis(cfg.contextLength, cfg.headSize, cfg.ropeTheta)
+
+
+def _blocks(tensors, role, cols, layer=0):
+    """Writable views of a Q8_0 matrix: the blocks' scales [row][block] and codes [row][block][32]."""
+    t, raw = tensors[(role, layer)]
+    tensors[(role, layer)] = (t, raw.copy())
+    b = tensors[(role, layer)][1].view(np.dtype([("d", np.float16), ("q", np.int8, 32)])).reshape(-1, cols // 32)
+    return b["d"], b["q"]
+
+
+def _scaled(query, key, heads=slice(None)):
+    """Query rows of these heads, and all key rows, times a power of two."""
+    def edit(cfg, tensors):
+        d, _ = _blocks(tensors, TensorRole.ATTENTION_QUERY, cfg.dim)
+        rows = d.reshape(cfg.numberOfHeads, cfg.headSize, -1)
+        rows[heads] = rows[heads].astype(np.float32) * np.float32(query)
+        d, _ = _blocks(tensors, TensorRole.ATTENTION_KEY, cfg.dim)
+        d[:] = d.astype(np.float32) * np.float32(key)
+    return edit
 
 
 @pytest.mark.parametrize("heads,kv_heads,head", [(4, 4, 64), (8, 4, 64), (8, 2, 64), (8, 1, 64), (2, 2, 128), (4, 2, 128), (8, 2, 128), (8, 1, 128)])
@@ -69,7 +96,23 @@ def test_many_ranges_pages_and_rows(dev, page, depths, width):
     assert max(errors) < BAR, errors
 
 
-def test_queries_beyond_binary16(dev):
-    """Query weights of a size that takes the rotated query past 65504: the kernel scales it before it is split."""
-    errors = attention_errors(dev, _rope, 4, 1, 64, 16, [3, 70], std=40.0)
-    assert all(np.isfinite(errors)) and max(errors) < 1e-3, errors  # scores of 1e5 and more: their last bits decide
+@pytest.mark.parametrize("heads,kv_heads,head", [(4, 4, 64), (8, 2, 64), (8, 1, 64), (8, 2, 128), (8, 1, 128)])
+@pytest.mark.parametrize("query,key", [(2.0 ** -6, 2.0 ** 6), (2.0 ** -12, 2.0 ** 12), (2.0 ** 15, 2.0 ** -13)])
+def test_queries_of_every_magnitude(dev, heads, kv_heads, head, query, key):
+    """Small queries against large keys, and queries beyond binary16 against small ones: scores of the same size as ever (four times
+    it in the last case), so the same bar: a query keeps its bits whatever its magnitude."""
+    outs = attention_outputs(dev, _rope, heads, kv_heads, head, 16, [3, 70, 300], edit=_scaled(query, key))
+    most = max(float(np.abs(q).max()) for _, _, q in outs)
+    assert most > 65504 if query > 1 else most < 8 * query, most
+    errors = [rel_l2(got.reshape(-1), want.reshape(-1)) for got, want, _ in outs]
+    assert max(errors) < BAR, errors
+
+
+@pytest.mark.parametrize("heads,kv_heads,head", [(8, 4, 64), (8, 2, 64), (8, 1, 64), (8, 2, 128), (8, 1, 128)])
+def test_large_head_beside_ordinary_ones(dev, heads, kv_heads, head):
+    """The heads that share a KV head with one whose query is 2^25 times as large lose nothing by it."""
+    group = heads // kv_heads
+    for got, want, q in attention_outputs(dev, _rope, heads, kv_heads, head, 16, [3, 70, 300], edit=_scaled(2.0 ** 25, 1.0, slice(0, None, group))):
+        assert np.abs(q[::group]).max() > 65504 and np.isfinite(got).all()
+        errors = [rel_l2(got[h], want[h]) for h in range(heads) if h % group != 0]
+        assert max(errors) < BAR, errors
