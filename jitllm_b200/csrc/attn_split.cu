@@ -13,7 +13,7 @@
 // keys per CTA as long as there are CTAs, then longer ranges. The last CTA of a (row, KV head) to finish folds the ranges'
 // results; the arrival is one atomic.
 // Error against a 64-bit softmax over the same query, keys and values (2-norm; geometric mean over 20 models, head sizes 64
-// and 128, groups of 2, 4 and 8, scores of standard deviation 0.2 to 8, 1 to 3000 keys): 1.47e-7; scalar binary32 sums in the
+// and 128, groups of 2, 4 and 8, scores of standard deviation 0.2 to 8, 1 to 3000 keys): 1.46e-7; scalar binary32 sums in the
 // split of the keys that a kernel of scalar products would take 1.50e-7. It does not depend on the size of the queries
 // (2^-12 to 2^15 times the usual one: 2.4e-7 to 2.7e-7 where it is 2.5e-7), nor on how the heads of a group compare.
 #include "ops.cuh"
@@ -418,6 +418,13 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
     if (!sm.is_last) return;
     for (int idx = tid; idx < G * nsplit; idx += kThreads) sm.fold[idx] = __ldcg(parts + size_t(idx) * ROW + HD);  // [range][head]
     // this thread's output elements in the first ranges, on their way meanwhile
+    auto weighted_pairs = [](const auto &x, const float *w) {  // the sum of x[i] w[i G]
+        constexpr int N = sizeof(x) / sizeof(float);
+        float s[N / 2];
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) s[i] = fmaf(x[2 * i + 1], w[(2 * i + 1) * G], x[2 * i] * w[2 * i * G]);
+        return sum_pairs(s);
+    };
     constexpr int kOut = (G * HD + kThreads - 1) / kThreads, kEarly = 4;
     float mine[kOut][kEarly];
 #pragma unroll
@@ -428,6 +435,8 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
     }
     __syncthreads();
     if (warp < G) {
+        // no weight for what fills up the first batch of loads, or the last one
+        if (lane < 12) sm.fold[(nsplit + lane) * G + warp] = 0.f;
         float M = -INFINITY;
         for (int s = lane; s < nsplit; s += 32) M = fmaxf(M, sm.fold[s * G + warp]);
         M = warp_max(M);
@@ -447,18 +456,12 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
         const int idx = tid + r * kThreads;
         if (idx >= G * HD) break;
         const int g = idx / HD, d = idx - g * HD;
-        float early[kEarly];
-#pragma unroll
-        for (int s = 0; s < kEarly; ++s) early[s] = s < nsplit ? mine[r][s] * sm.fold[s * G + g] : 0.f;
-        float val = sum_pairs(early);
+        float val = weighted_pairs(mine[r], &sm.fold[g]);
         for (int s0 = kEarly; s0 < nsplit; s0 += 8) {
             float more[8];
 #pragma unroll
             for (int s = 0; s < 8; ++s) more[s] = s0 + s < nsplit ? __ldcg(parts + (size_t(s0 + s) * G + g) * ROW + d) : 0.f;
-#pragma unroll
-            for (int s = 0; s < 8; ++s)
-                if (s0 + s < nsplit) more[s] *= sm.fold[(s0 + s) * G + g];
-            val += sum_pairs(more);
+            val += weighted_pairs(more, &sm.fold[s0 * G + g]);
         }
         attn_store(a, size_t(b), (kvh * G + g) * HD + d, val * sm.inv[g]);
     }
@@ -471,7 +474,8 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
 
 template <int HD, int G>
 cudaError_t launch_t(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic) {
-    if (a.nsplit < 1 || a.nsplit * G > 1024) return cudaErrorInvalidValue;  // the fold's table
+    static_assert((kAttnMaxSplits + 12) * G <= 1024, "the fold's table");
+    if (a.nsplit < 1 || a.nsplit > kAttnMaxSplits) return cudaErrorInvalidValue;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(a.nsplit, a.kv_heads, width);
     cfg.blockDim = dim3(kThreads);
