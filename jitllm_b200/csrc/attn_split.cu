@@ -101,8 +101,63 @@ struct SplitAttn {
     };
 };
 
+// The CTA's range once more, in scalar binary32, when an infinity or NaN showed in its output: a zero part of a query or
+// probability, or a row of the tile that holds no part, makes NaN of an infinite key or value, and so do parts of opposite signs.
+// Here, as in the reference, a score of -inf has no weight, an infinite value gives an infinite output, and a NaN score reaches the
+// output. Its speed matters to nobody: keys beyond 65504 do not occur in a model that works. Warp w takes every fourth key for
+// half of the heads; the results go to the merge area as the tiles' do. Ends with that area written, no barrier.
 template <int HD, int G>
-__global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs a) {
+__device__ __forceinline__ void scalar_range(const AttnArgs &a, typename SplitAttn<HD, G>::Smem &sm, int b, int kvh, int pos, int slot, int start, int end) {
+    constexpr int PAIRS = HD / 64;  // pairs of dimensions per lane
+    const int lane = threadIdx.x & 31, kg = (threadIdx.x >> 5) % kGroups, half = (threadIdx.x >> 5) / kGroups;
+    const int bt = a.kv.block_tokens, kv_dim = a.kv.kv_dim;
+    const int32_t *table = a.kv.block_table + int64_t(slot) * a.kv.blocks_per_slot;
+    const float inv_sqrt = 1.0f / sqrtf(static_cast<float>(HD));
+    for (int g = half; g < G; g += 2) {
+        float2 q[PAIRS], o[PAIRS];
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            const int p = lane + 32 * i;
+            const float2 x = __ldcg(reinterpret_cast<const float2 *>(a.q + size_t(b) * a.dim + size_t(kvh * G + g) * HD) + p);
+            const float c = a.rope_cos[size_t(pos) * (HD / 2) + p], s = a.rope_sin[size_t(pos) * (HD / 2) + p];
+            q[i] = make_float2(__fsub_rn(__fmul_rn(x.x, c), __fmul_rn(x.y, s)), __fadd_rn(__fmul_rn(x.x, s), __fmul_rn(x.y, c)));
+            o[i] = make_float2(0.f, 0.f);
+        }
+        float m = -INFINITY, l = 0.f;
+        for (int t = start + kg; t < end; t += kGroups) {
+            const int64_t off = ((int64_t(table[t / bt]) * a.kv.layers + a.layer) * bt + t % bt) * kv_dim + int64_t(kvh) * HD;
+            float2 v[PAIRS];
+            float s = 0.f;
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                const float2 k = __half22float2(__ldcg(reinterpret_cast<const __half2 *>(a.kv.kpool + off) + lane + 32 * i));
+                v[i] = __half22float2(__ldcg(reinterpret_cast<const __half2 *>(a.kv.vpool + off) + lane + 32 * i));
+                s += q[i].x * k.x + q[i].y * k.y;
+            }
+            s = warp_sum(s) * inv_sqrt;
+            const float mn = fmaxf(m, s), corr = mn == -INFINITY ? 1.0f : expf(m - mn), p = s == -INFINITY ? 0.f : expf(s - mn);
+            m = mn;
+            l = l * corr + p;
+#pragma unroll
+            for (int i = 0; i < PAIRS; ++i) {
+                o[i].x = o[i].x * corr + p * v[i].x;
+                o[i].y = o[i].y * corr + p * v[i].y;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < PAIRS; ++i) {
+            sm.merge[kg][g][2 * (lane + 32 * i)] = o[i].x;
+            sm.merge[kg][g][2 * (lane + 32 * i) + 1] = o[i].y;
+        }
+        if (lane == 0) {
+            sm.merge[kg][g][HD] = m;
+            sm.merge[kg][g][HD + 1] = l;
+        }
+    }
+}
+
+template <int HD, int G>
+__global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const __grid_constant__ AttnArgs a) {
     using A = SplitAttn<HD, G>;
     constexpr int LD = A::LD, QT = A::QT, DB = HD / 16, ROW = HD + 2, PARTS = HD / 8;
     extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -298,14 +353,14 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
         const float mn = fmaxf(m, top);
-        // every score of the group may be -inf (an infinite query or key): no weight, as the reference's exp(-inf - max)
+        // a score of -inf (an infinite key, or a masked one) has no weight, also when there is no larger one yet; NaN stays
         const float corr = mn == -INFINITY ? 1.0f : expf(m - mn);
         m = mn;
         uint32_t pf[QT][4];
         __half part[4][3];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            s[c] = mn == -INFINITY ? 0.f : expf(s[c] - mn);
+            s[c] = s[c] == -INFINITY ? 0.f : expf(s[c] - mn);
             split3(s[c] * kUp, part[c]);
         }
         l = fmaf(l, corr, (s[0] + s[1]) + (s[2] + s[3]));
@@ -352,9 +407,12 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
     __syncthreads();  // everybody is done with the tiles: their memory becomes the merge area
+    float all[2] = {0.f, 0.f};  // sums of this thread's outputs: infinite or NaN when one is
 #pragma unroll
     for (int d = 0; d < DB; ++d) {
         const float x = join(o[d][0] + o[d][2]), y = join(o[d][1] + o[d][3]);
+        all[0] += x;
+        all[1] += y;
         if (gl < G) {
             sm.merge[kg][gl][half * (HD / 2) + d * 8 + 2 * t] = x * (1.0f / kUp);
             sm.merge[kg][gl][half * (HD / 2) + d * 8 + 2 * t + 1] = y * (1.0f / kUp);
@@ -364,7 +422,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const AttnArgs 
         sm.merge[kg][gl][HD] = m;
         sm.merge[kg][gl][HD + 1] = l;
     }
-    __syncthreads();
+    // (a NaN score makes all outputs of its head NaN, so that they show it)
+    if (__builtin_expect(__syncthreads_or(!(fabsf(all[0] + all[1]) < INFINITY)), 0)) {
+        scalar_range<HD, G>(a, sm, b, kvh, pos, slot, start, end);
+        __syncthreads();
+    }
     if (tid < G * kGroups) {  // four lanes per head: the groups' maxima and sums (one without keys weighs nothing)
         const int g = tid / kGroups, w = tid % kGroups;
         const unsigned lanes = G * kGroups >= 32 ? 0xffffffffu : (1u << (G * kGroups)) - 1u;

@@ -1,7 +1,7 @@
 """Decode attention with the keys split over CTAs, by itself: the attention output of a one-layer model's step against a 64-bit
 softmax over the query, keys and values that the device itself used (the projections and pages are read back), at the depths
 where the split changes: one key, around one tile of 64, where a second range, a third and the last of twenty begin, and
-where ranges grow beyond a tile; every head size and group; queries of every magnitude."""
+where ranges grow beyond a tile; every head size and group; queries of every magnitude; infinities and NaN among keys and values."""
 import numpy as np
 import pytest
 
@@ -15,9 +15,9 @@ pytestmark = pytest.mark.gpu
 BAR = 1e-5
 
 
-def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, std=0.05, seed=3, edit=None):
+def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, std=0.05, seed=3, edit=None, special=None, token=5):
     """(output, 64-bit output, rotated query), [head][dimension] each, of one step at every depth (keys in the pages before it).
-    `edit` changes the tensors."""
+    `edit` changes the tensors, `special` the prompt ({position: token}), `token` is what row 0's step takes in."""
     cfg = jl.Configuration(dim=heads * head, hiddenDim=512, numberOfLayers=1, numberOfHeads=heads, numberOfKeyValueHeads=kv_heads,
                            vocabularySize=512, contextLength=max(depths) + 16)
     tensors = jl.synth_model_tensors(cfg, GGMLType.Q8_0, seed=seed, std=std)
@@ -30,7 +30,9 @@ def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, s
     kv.publishBlockTable(np.random.default_rng(seed).permutation(width * bps).astype(np.int32))
     kv.fill(0x7E00)  # NaN wherever nothing was written
     rng = np.random.default_rng(seed + 1)
-    prompt = rng.integers(0, cfg.vocabularySize, size=max(depths)).astype(np.int32)
+    prompt = rng.integers(3, cfg.vocabularySize, size=max(depths)).astype(np.int32)
+    for at, what in (special or {}).items():
+        prompt[at] = what
     for b in range(width):
         jl.B200InvocationBoundary(model, kvSlot=b).prefill(prompt if max(depths) > 0 else [1], 0)
     ex = jl.B200BatchExecutor(model)
@@ -38,7 +40,7 @@ def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, s
     out = []
     for pos in sorted(depths, reverse=True):  # the step overwrites the key at its position: deepest first
         rows = [max(0, pos - 3 * b) for b in range(width)]
-        ex.decodeStep(jl.BatchSlots([True] * width, [5 + b for b in range(width)], rows, list(range(width))))
+        ex.decodeStep(jl.BatchSlots([True] * width, [token + b for b in range(width)], rows, list(range(width))))
         for b, p in enumerate(rows):
             q = model.debugRead("q", b).reshape(heads, head // 2, 2)
             q = np.stack([q[..., 0] * cr[p] - q[..., 1] * ci[p], q[..., 0] * ci[p] + q[..., 1] * cr[p]], axis=-1)
@@ -47,10 +49,11 @@ def attention_outputs(dev, rope, heads, kv_heads, head, page, depths, width=1, s
                     for w in ("k", "v"))
             got = model.debugRead("xb", b).reshape(heads, head)
             want = np.empty((heads, head))
-            for h in range(heads):
-                s = k[:, h * kv_heads // heads] @ q[h] / np.sqrt(head)
-                w = np.exp(s - s.max())
-                want[h] = (w / w.sum()) @ v[:, h * kv_heads // heads]
+            with np.errstate(invalid="ignore"):
+                for h in range(heads):
+                    s = k[:, h * kv_heads // heads] @ q[h] / np.sqrt(head)
+                    w = np.exp(s - s.max())
+                    want[h] = (w / w.sum()) @ v[:, h * kv_heads // heads]
             out.append((got, want, q))
     kv.close()
     return out
@@ -116,3 +119,63 @@ def test_large_head_beside_ordinary_ones(dev, heads, kv_heads, head):
         assert np.abs(q[::group]).max() > 65504 and np.isfinite(got).all()
         errors = [rel_l2(got[h], want[h]) for h in range(heads) if h % group != 0]
         assert max(errors) < BAR, errors
+
+
+KEY, VALUE = 1, 2  # tokens whose key (value) goes beyond binary16 in some components: infinite in the pages
+
+
+def _overflow(cfg, tensors):
+    """Embedding columns 0 and 32 are zero for all tokens but KEY and VALUE; key component 0 and value component 5 of every KV head
+    weigh these columns with more than 6e4."""
+    d, q = _blocks(tensors, TensorRole.TOKEN_EMBEDDING, cfg.dim, -1)
+    q[:, 0:2, 0] = 0
+    for block, token in ((0, KEY), (1, VALUE)):
+        d[token, block], q[token, block] = 1.0, 0
+        q[token, block, 0] = 127
+    for role, block, component in ((TensorRole.ATTENTION_KEY, 0, 0), (TensorRole.ATTENTION_VALUE, 1, 5)):
+        d, q = _blocks(tensors, role, cfg.dim)
+        rows = slice(component, None, cfg.headSize)
+        d[rows, block], q[rows, block] = 500.0, 0
+        q[rows, block, 0] = 127
+
+
+@pytest.mark.parametrize("heads,kv_heads,head", [(8, 8, 64), (8, 4, 64), (8, 2, 64), (8, 1, 64), (8, 4, 128), (8, 2, 128), (8, 1, 128)])
+@pytest.mark.parametrize("pos,special,token", [
+    (70, {0: KEY}, 5),        # scores of +inf (the output is NaN) or -inf (no weight) by the sign of the query
+    (300, {101: KEY}, 5),     # the same, or NaN, in one of five ranges
+    (66, {32: KEY}, 5),       # the same, the only key of a warp's sixteen
+    (16, {}, KEY),            # the same, the step's own key
+    (300, {101: VALUE}, 5),   # an output of +-inf
+    (16, {}, VALUE),
+    (130, {3: KEY, 127: VALUE}, 5)])
+def test_infinite_keys_and_values(dev, heads, kv_heads, head, pos, special, token):
+    outs = []
+    for seed in (3, 4, 5):
+        outs += attention_outputs(dev, _rope, heads, kv_heads, head, 16, [pos], seed=seed, edit=_overflow, special=special, token=token)
+    keys = KEY in special.values() or token == KEY
+    values = VALUE in special.values() or token == VALUE
+    nan = np.concatenate([np.isnan(want).all(axis=1) for _, want, _ in outs])
+    assert not keys or (nan.any() and not nan.all())
+    assert not values or any(np.isinf(want[:, 5]).any() for _, want, _ in outs)
+    for got, want, _ in outs:
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        inf = np.isinf(want)
+        assert np.array_equal(got[inf], want[inf])
+        for h in range(heads):
+            fine = np.isfinite(want[h])
+            assert not fine.any() or rel_l2(got[h][fine], want[h][fine]) < BAR
+
+
+def test_nan_key(dev):
+    """Positions that nothing was written to hold NaN: an output that attends to one is NaN."""
+    cfg = jl.Configuration(dim=512, hiddenDim=512, numberOfLayers=1, numberOfHeads=8, numberOfKeyValueHeads=2, vocabularySize=512, contextLength=128)
+    model = jl.load_model(dev, cfg, jl.synth_model_tensors(cfg, GGMLType.Q8_0, seed=3, std=0.05), *_rope(cfg))
+    kv = model.createKvStorage(jl.KvStorageRequest(8, 8, 1, 16, 1, cfg.kvDim))
+    kv.publishBlockTable(np.arange(8, dtype=np.int32))
+    kv.fill(0x7E00)
+    boundary = jl.B200InvocationBoundary(model, kvSlot=0)
+    boundary.prefill(np.arange(32, dtype=np.int32), 0)
+    boundary.prefill(np.arange(33, 65, dtype=np.int32), 33)
+    jl.B200BatchExecutor(model).decodeStep(jl.BatchSlots([True], [5], [65], [0]))
+    assert np.isnan(model.debugRead("xb")).all()
+    kv.close()
