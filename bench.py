@@ -682,7 +682,7 @@ def main():
         "scaling": "weak" if replicas > 1 else "strong", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic", "config": config, "parallelism": parallelism,
         "clocks": clocks,
-        "e2e": {"value": tokens * replicas / (e_ms / 1000.0), "unit": "tok/s", "h2d_bytes_per_step": 13 * B,
+        "e2e": {"value": tokens * replicas / (e_ms / 1000.0), "unit": "tok/s", "h2d_bytes_per_step": 16 * B,
                 "d2h_bytes_per_step": 4 * B + 4, "ms_per_step": e_ms / K},
         "gpu_launches": int(c1["kernel_launches"] - c0["kernel_launches"]),
         "roofline": {"bound": "hbm", "kernel": "gemv_kernel<%s> %s" % (args.format, dom["kernel"]),

@@ -138,8 +138,7 @@ struct jl_ctx {
     float *d_uniforms = nullptr;            // jl_sample: one random number per row
     int batch_attn_min_pairs = 0;           // (rows x KV heads) from which decode batches use attention_batch_launch
     int logits_rows = 0;                    // rows of ctx->logits the last jl_decode left valid
-    // pinned host staging: tokens | positions | slots | out | active | status
-    int32_t *h_stage = nullptr;
+    int32_t *h_stage = nullptr;  // pinned host staging (StepStage)
 
     std::map<int, StepGraph> graphs;  // key: width
     uint32_t *flush_buf = nullptr;
@@ -1166,8 +1165,26 @@ cudaError_t clear_after_timeout(jl_ctx *ctx) {
     return e;
 }
 
+// The pinned staging words: a step's inputs, four arrays row_cap words apart as they lie on the device (upload_rows copies them
+// as one), then what comes back.
+struct StepStage {
+    int32_t *tokens, *positions, *slots;
+    uint8_t *active;
+    int32_t *out, *status;
+    explicit StepStage(const jl_ctx *ctx) {
+        const size_t B = ctx->row_cap;
+        tokens = ctx->h_stage;
+        positions = tokens + B;
+        slots = positions + B;
+        active = reinterpret_cast<uint8_t *>(slots + B);
+        out = ctx->h_stage + 4 * B;
+        status = ctx->h_stage + 5 * B;
+    }
+};
+constexpr int kInputRowBytes = 16;  // of a step's inputs per row: the active flag takes a word of its own
+
 int check_status(jl_ctx *ctx) {
-    int st = ctx->h_stage[5 * ctx->row_cap];
+    int st = *StepStage(ctx).status;
     if (st == kDevTimeout) {
         JL_CUDA(ctx, clear_after_timeout(ctx));
         return fail(ctx, JL_ERR_TIMEOUT, "a kernel gave up waiting for an asynchronous copy");
@@ -1644,8 +1661,8 @@ int32_t jl_kv_read_row(jl_ctx *ctx, int32_t which, int32_t slot, int32_t layer, 
 }
 
 // The inputs of a step of n rows, from the staging words to the device, in one copy: four rows (tokens, positions, slots,
-// active flags) of 4 n bytes, row_cap words apart on both sides. (Four copies cost a step 6 us more: a small model's step with
-// its logits 173.0 -> 166.7 us.)
+// active flags) of 4 n bytes, row_cap words apart on both sides. (A small model's step with its logits: 166.7 us, with four
+// copies 173.0.)
 static cudaError_t upload_rows(jl_ctx *ctx, int n) {
     const size_t pitch = size_t(ctx->row_cap) * 4;
     return cudaMemcpy2DAsync(ctx->d_tokens, pitch, ctx->h_stage, pitch, size_t(n) * 4, 4, cudaMemcpyHostToDevice, ctx->stream);
@@ -1685,19 +1702,16 @@ int32_t jl_decode(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int32
     int rc = validate_rows(ctx, width, tokens, positions, kv_slots, active);
     if (rc) return rc;
     cudaSetDevice(ctx->device);
-    const size_t B = ctx->row_cap;
-    int32_t *h_tok = ctx->h_stage, *h_pos = h_tok + B, *h_slot = h_pos + B, *h_out = ctx->h_stage + 4 * B;
-    uint8_t *h_act = reinterpret_cast<uint8_t *>(h_slot + B);
-    int32_t *h_status = ctx->h_stage + 5 * B;
+    const StepStage h(ctx);
     for (int b = 0; b < width; ++b) {
         const bool on = !active || active[b];
-        h_tok[b] = on ? tokens[b] : 0;
-        h_pos[b] = on ? positions[b] : 0;
-        h_slot[b] = on ? kv_slots[b] : 0;
-        h_act[b] = on ? 1 : 0;
+        h.tokens[b] = on ? tokens[b] : 0;
+        h.positions[b] = on ? positions[b] : 0;
+        h.slots[b] = on ? kv_slots[b] : 0;
+        h.active[b] = on ? 1 : 0;
     }
     bool any = false;
-    for (int b = 0; b < width; ++b) any = any || h_act[b];
+    for (int b = 0; b < width; ++b) any = any || h.active[b];
     if (!any) {
         for (int b = 0; b < width; ++b) out_tokens[b] = -1;
         return JL_OK;
@@ -1705,8 +1719,8 @@ int32_t jl_decode(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int32
     JL_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     JL_CUDA(ctx, upload_rows(ctx, width));
     if ((rc = run_step(ctx, width, true, false))) return rc;
-    JL_CUDA(ctx, cudaMemcpyAsync(h_out, ctx->d_out, width * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    JL_CUDA(ctx, cudaMemcpyAsync(h_status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    JL_CUDA(ctx, cudaMemcpyAsync(h.out, ctx->d_out, width * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    JL_CUDA(ctx, cudaMemcpyAsync(h.status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
     std::vector<float> gathered;
     if (out_logits && ctx->tp_size > 1) {
         // Every rank holds [row][l_vocab]; gather them as [rank][row][l_vocab] and let the host
@@ -1725,7 +1739,7 @@ int32_t jl_decode(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int32
     JL_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     JL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
-    for (int b = 0; b < width; ++b) out_tokens[b] = h_act[b] ? h_out[b] : -1;
+    for (int b = 0; b < width; ++b) out_tokens[b] = h.active[b] ? h.out[b] : -1;
     if (out_logits && ctx->tp_size > 1) {
         for (int k = 0; k < ctx->tp_size; ++k)
             for (int b = 0; b < width; ++b)
@@ -1735,7 +1749,7 @@ int32_t jl_decode(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int32
     cudaEventElapsedTime(&ctx->counters.last_step_ms, ctx->ev0, ctx->ev1);
     ctx->logits_rows = width;
     ctx->counters.decode_calls++;
-    ctx->counters.h2d_bytes += width * 13;
+    ctx->counters.h2d_bytes += size_t(width) * kInputRowBytes;
     ctx->counters.d2h_bytes += width * 4 + 4 + (out_logits ? size_t(width) * ctx->desc.vocab * 4 : 0);
     return JL_OK;
 }
@@ -1761,8 +1775,8 @@ int32_t jl_sample(jl_ctx *ctx, int32_t width, float temperature, float topp, con
         ctx->user_allocs.push_back(ctx->d_uniforms);  // released with the context
         JL_CUDA(ctx, sample_rows_configure());
     }
-    float *h_u = reinterpret_cast<float *>(ctx->h_stage);
-    int32_t *h_out = ctx->h_stage + 3 * size_t(ctx->row_cap);
+    const StepStage h(ctx);
+    float *h_u = reinterpret_cast<float *>(h.tokens);
     memcpy(h_u, uniforms, size_t(width) * 4);
     JL_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     JL_CUDA(ctx, cudaMemcpyAsync(ctx->d_uniforms, h_u, size_t(width) * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -1770,10 +1784,10 @@ int32_t jl_sample(jl_ctx *ctx, int32_t width, float temperature, float topp, con
                                        ctx->d_out, ctx->d_out, ctx->stream);  // d_out: the step's arg-max in, the sample out
     if (e != cudaSuccess) return fail(ctx, JL_ERR_CUDA, "sampling launch failed: %s", cudaGetErrorString(e));
     ctx->counters.kernel_launches += 1;
-    JL_CUDA(ctx, cudaMemcpyAsync(h_out, ctx->d_out, size_t(width) * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    JL_CUDA(ctx, cudaMemcpyAsync(h.out, ctx->d_out, size_t(width) * 4, cudaMemcpyDeviceToHost, ctx->stream));
     JL_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     JL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int b = 0; b < width; ++b) out_tokens[b] = h_out[b];
+    for (int b = 0; b < width; ++b) out_tokens[b] = h.out[b];
     cudaEventElapsedTime(&ctx->counters.last_step_ms, ctx->ev0, ctx->ev1);
     ctx->logits_rows = 0;  // the rows now hold exp(score - max), not logits
     ctx->counters.h2d_bytes += size_t(width) * 4;
@@ -1789,10 +1803,7 @@ int32_t jl_prefill(jl_ctx *ctx, int32_t kv_slot, const int32_t *tokens, int32_t 
                "tokens must not be NULL, n and start_pos must not be negative");
     if (n == 0) return JL_OK;
     cudaSetDevice(ctx->device);
-    const size_t B = ctx->row_cap;
-    int32_t *h_tok = ctx->h_stage, *h_pos = h_tok + B, *h_slot = h_pos + B, *h_out = ctx->h_stage + 4 * B;
-    uint8_t *h_act = reinterpret_cast<uint8_t *>(h_slot + B);
-    int32_t *h_status = ctx->h_stage + 5 * B;
+    const StepStage h(ctx);
     JL_CUDA(ctx, cudaEventRecord(ctx->ev0, ctx->stream));
     {
         const int32_t first = tokens[0], last_pos = start_pos + n - 1;
@@ -1814,10 +1825,10 @@ int32_t jl_prefill(jl_ctx *ctx, int32_t kv_slot, const int32_t *tokens, int32_t 
         if (chunk > ctx->row_cap) chunk = ctx->row_cap;
         if (chunk < rows_min) chunk = 1;
         for (int i = 0; i < chunk; ++i) {
-            h_tok[i] = tokens[done + i];
-            h_pos[i] = start_pos + done + i;
-            h_slot[i] = kv_slot;
-            h_act[i] = 1;
+            h.tokens[i] = tokens[done + i];
+            h.positions[i] = start_pos + done + i;
+            h.slots[i] = kv_slot;
+            h.active[i] = 1;
         }
         JL_CUDA(ctx, upload_rows(ctx, chunk));
         int rc;
@@ -1833,14 +1844,14 @@ int32_t jl_prefill(jl_ctx *ctx, int32_t kv_slot, const int32_t *tokens, int32_t 
         JL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
         done += chunk;
     }
-    JL_CUDA(ctx, cudaMemcpyAsync(h_status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    JL_CUDA(ctx, cudaMemcpyAsync(h.status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
     JL_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     JL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     int rc = check_status(ctx);
     if (rc) return rc;
     cudaEventElapsedTime(&ctx->counters.last_step_ms, ctx->ev0, ctx->ev1);
     ctx->counters.prefill_calls++;
-    ctx->counters.h2d_bytes += size_t(n) * 13;
+    ctx->counters.h2d_bytes += size_t(n) * kInputRowBytes;
     return JL_OK;
 }
 
@@ -1877,19 +1888,16 @@ int32_t jl_generate(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int
         ctx->history_cap = need;
     }
     if (!ctx->d_step && (rc = dev_alloc(ctx, reinterpret_cast<void **>(&ctx->d_step), 4))) return rc;
-    const size_t B = ctx->row_cap;
-    int32_t *h_tok = ctx->h_stage, *h_pos = h_tok + B, *h_slot = h_pos + B, *h_out = ctx->h_stage + 4 * B;
-    uint8_t *h_act = reinterpret_cast<uint8_t *>(h_slot + B);
-    int32_t *h_status = ctx->h_stage + 5 * B;
+    const StepStage h(ctx);
     for (int b = 0; b < width; ++b) {
         const bool on = !active || active[b];
-        h_tok[b] = on ? tokens[b] : 0;
-        h_pos[b] = on ? positions[b] : 0;
-        h_slot[b] = on ? kv_slots[b] : 0;
-        h_act[b] = on ? 1 : 0;
+        h.tokens[b] = on ? tokens[b] : 0;
+        h.positions[b] = on ? positions[b] : 0;
+        h.slots[b] = on ? kv_slots[b] : 0;
+        h.active[b] = on ? 1 : 0;
     }
     bool any = false;
-    for (int b = 0; b < width; ++b) any = any || h_act[b];
+    for (int b = 0; b < width; ++b) any = any || h.active[b];
     if (!any) {
         for (size_t i = 0; i < need; ++i) out_history[i] = -1;
         return JL_OK;
@@ -1900,13 +1908,13 @@ int32_t jl_generate(jl_ctx *ctx, int32_t width, const int32_t *tokens, const int
     for (int s = 0; s < n_steps; ++s)
         if ((rc = run_step(ctx, width, true, true))) return rc;
     JL_CUDA(ctx, cudaMemcpyAsync(out_history, ctx->d_history, need * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    JL_CUDA(ctx, cudaMemcpyAsync(h_status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
+    JL_CUDA(ctx, cudaMemcpyAsync(h.status, ctx->d_status, 4, cudaMemcpyDeviceToHost, ctx->stream));
     JL_CUDA(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
     JL_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
     cudaEventElapsedTime(&ctx->counters.last_step_ms, ctx->ev0, ctx->ev1);
     ctx->counters.decode_calls += n_steps;
-    ctx->counters.h2d_bytes += width * 13;
+    ctx->counters.h2d_bytes += size_t(width) * kInputRowBytes;
     ctx->counters.d2h_bytes += need * 4 + 4;
     return JL_OK;
 }
