@@ -100,7 +100,6 @@ struct jl_ctx {
     int *amax_idx = nullptr;
     unsigned *amax_count = nullptr;
     int *d_status = nullptr;
-    int attn_nsplit = 1;
     // tensor-parallel placement: local (per-GPU) extents of the sharded dimensions
     int tp_rank = 0, tp_size = 1;
     int l_heads = 0, l_kv_heads = 0, l_qdim = 0, l_hidden = 0, l_vocab = 0;
@@ -1509,7 +1508,6 @@ int32_t jl_model_finalize(jl_ctx *ctx) {
         const size_t v = size_t(w) * size_t(attn_splits_for_width(ctx, w));
         if (v > max_row_splits) max_row_splits = v;
     }
-    ctx->attn_nsplit = attn_splits_for_width(ctx, 1);
     if ((rc = alloc(reinterpret_cast<void **>(&ctx->x), R * d.dim * 4))) return rc;
     if ((rc = alloc(reinterpret_cast<void **>(&ctx->q), R * ctx->l_qdim * 4))) return rc;
     if ((rc = alloc(reinterpret_cast<void **>(&ctx->k), R * ctx->kv_dim * 4))) return rc;
