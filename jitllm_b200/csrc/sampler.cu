@@ -38,7 +38,9 @@ constexpr int kMaxCluster = 8;
 constexpr int kSampleThreads = 1024;
 constexpr int kSampleWarps = kSampleThreads / 32;
 constexpr int kBuckets = 2048;
-constexpr int kKeep = 16;  // elements a thread keeps in registers between the passes (8 x 1024 x 16 = 131 072 per row)
+// Elements a thread keeps in registers between the passes: all of a row of up to C x 16 384 elements with C CTAs. At 128 256
+// tokens that is every element with eight CTAs, half of them with four and a quarter with two; the others are read again (from L2).
+constexpr int kKeep = 16;
 
 __device__ __forceinline__ unsigned long long to_fixed(float e) {
     return static_cast<unsigned long long>(__float2ull_rz(e * 1099511627776.0f));  // exact scaling by 2^40
@@ -135,7 +137,7 @@ __device__ __forceinline__ void hist_add(SampleSmem &sm, int bucket, unsigned lo
 }
 
 // The first kKeep elements of a thread (element lo + rd * 1024 + tid for round rd) stay in registers after the
-// exponential pass, so the later passes of a row of up to 131 072 tokens read nothing from memory.
+// exponential pass, the later ones are read from the row again in every pass.
 __device__ void hist_pass(const float *e, const float (&kept)[kKeep], int lo, int hi, unsigned prefix, int known, int bits,
                           SampleSmem &sm) {
     const int nb = 1 << bits, shift = 31 - known - bits;
