@@ -513,19 +513,24 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const __grid_co
         if (lane == 0) sm.inv[warp] = 1.0f / L;
     }
     __syncthreads();
+    float val[kOut];
+#pragma unroll
+    for (int r = 0; r < kOut; ++r) val[r] = weighted_pairs(mine[r], &sm.fold[(tid + r * kThreads) / HD % G]);
+    for (int s0 = kEarly; s0 < nsplit; s0 += 8) {
+        float more[kOut][8];  // eight ranges of all of this thread's elements in flight
+#pragma unroll
+        for (int r = 0; r < kOut; ++r) {
+            const int idx = tid + r * kThreads;
+#pragma unroll
+            for (int s = 0; s < 8; ++s) more[r][s] = idx < G * HD && s0 + s < nsplit ? __ldcg(parts + (size_t(s0 + s) * G + idx / HD) * ROW + idx % HD) : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < kOut; ++r) val[r] += weighted_pairs(more[r], &sm.fold[s0 * G + (tid + r * kThreads) / HD % G]);
+    }
 #pragma unroll
     for (int r = 0; r < kOut; ++r) {
         const int idx = tid + r * kThreads;
-        if (idx >= G * HD) break;
-        const int g = idx / HD, d = idx - g * HD;
-        float val = weighted_pairs(mine[r], &sm.fold[g]);
-        for (int s0 = kEarly; s0 < nsplit; s0 += 8) {
-            float more[8];
-#pragma unroll
-            for (int s = 0; s < 8; ++s) more[s] = s0 + s < nsplit ? __ldcg(parts + (size_t(s0 + s) * G + g) * ROW + d) : 0.f;
-            val += weighted_pairs(more, &sm.fold[s0 * G + g]);
-        }
-        attn_store(a, size_t(b), (kvh * G + g) * HD + d, val * sm.inv[g]);
+        if (idx < G * HD) attn_store(a, size_t(b), kvh * (G * HD) + idx, val[r] * sm.inv[idx / HD]);
     }
     if (tid == 0) {
         *arrived = 0u;

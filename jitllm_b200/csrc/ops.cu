@@ -658,9 +658,14 @@ size_t attention_partial_floats(int width, int heads, int nsplit, int head_dim) 
 }
 
 int attention_splits(int sm_count, int width, int kv_heads) {
-    // About two CTAs per SM over the whole launch; a single CTA folds the ranges of a (row, KV head), so not more than
-    // kAttnMaxSplits of them.
-    return std::max(1, std::min(kAttnMaxSplits, 2 * sm_count / (width * kv_heads)));
+    // Not more than two CTAs per SM over the whole launch (launches of 16 pairs or more). Below that, twenty ranges, or as many
+    // as a CTA can fold in passing where few pairs would leave SMs without a CTA. A grid is sized for the longest context, and
+    // CTAs that find no keys of their own cost the short ones: a step of eight layers with 8 KV heads takes 284.0 us at 57 keys with
+    // 20 ranges, 285.7 with 28, 288.4 with 37 (at 8000 keys of head size 128: 539, 508, 507), five rows of one KV head (sixteen
+    // layers) 687 us at 300 keys with 20 and 710 with 32. With 2 KV heads the grid stays small: 432 us at 300 keys with 20, 28 and
+    // 37; 545, 521 and 510 at 4000, 891, 759 and 700 at 16000. Past 37 the fold eats the gain (48: 515 at 4000).
+    const int pairs = width * kv_heads;
+    return std::max(1, std::min(kAttnMaxSplits * pairs <= sm_count ? kAttnMaxSplits : 20, 2 * sm_count / pairs));
 }
 
 cudaError_t attention_batch_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic) {

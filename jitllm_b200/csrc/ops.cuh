@@ -28,7 +28,7 @@ struct AttnArgs {
     int layer, heads, kv_heads, head_dim, dim;
     int nsplit;  // from attention_splits()
     int append;  // 1: the CTA owning the new position rotates k and appends k,v; 0: pages already hold it
-    float *partial;     // scratch [width][heads][nsplit][head_dim + 2]
+    float *partial;     // scratch [width][kv_heads][nsplit][heads / kv_heads][head_dim + 2]
     unsigned *counters; // scratch [width][kv_heads], zero between launches
     int *status;        // device status word (attention_prompt_launch), nullable
 };
@@ -59,8 +59,8 @@ cudaError_t attention_prompt_launch(const AttnArgs &a, int n, cudaStream_t strea
 // query heads as the rows of a tensor-core tile; rotates and appends the step's own key and value itself.
 cudaError_t attention_batch_launch(const AttnArgs &a, int width, cudaStream_t stream, bool programmatic);
 size_t attention_partial_floats(int width, int heads, int nsplit, int head_dim);
-// Key ranges per (row, KV head), at most, for a launch of `width` rows.
-constexpr int kAttnMaxSplits = 20;
+// Key ranges per (row, KV head), at most, for a launch of `width` rows; in any launch not more than kAttnMaxSplits.
+constexpr int kAttnMaxSplits = 37;
 int attention_splits(int sm_count, int width, int kv_heads);
 
 // x[row] = getFloat of embedding row tokens[row] (inference/op/CpuOperations.java:30-32).

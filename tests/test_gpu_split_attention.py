@@ -1,7 +1,7 @@
 """Decode attention with the keys split over CTAs, by itself: the attention output of a one-layer model's step against a 64-bit
 softmax over the query, keys and values that the device itself used (the projections and pages are read back), at the depths
-where the split changes: one key, around one tile of 64, where a second range, a third and the last of twenty begin, and
-where ranges grow beyond a tile; every head size and group; queries of every magnitude; infinities and NaN among keys and values."""
+where the split changes: one key, around one tile of 64, where a second range, a third and the last of twenty (eight KV heads)
+or thirty-seven (two) begin, where the fold takes another batch of ranges, and where ranges grow beyond a tile; every head size and group; queries of every magnitude; infinities and NaN among keys and values."""
 import numpy as np
 import pytest
 
@@ -96,6 +96,14 @@ def test_range_and_tile_edges(dev, heads, kv_heads, head):
 @pytest.mark.parametrize("page,depths,width", [(16, [1279, 1280, 1281, 2600], 1), (1, [700, 1281], 1), (16, [300, 900], 3)])
 def test_many_ranges_pages_and_rows(dev, page, depths, width):
     errors = attention_errors(dev, _rope, 8, 2, 64, page, depths, width)
+    assert max(errors) < BAR, errors
+
+
+@pytest.mark.parametrize("heads,kv_heads,head,depths", [
+    (8, 2, 64, [255, 256, 257, 767, 768, 769, 1791, 1792, 1793, 2303, 2304, 2305, 2367, 2368, 2369]), (8, 8, 64, [1279, 1280, 1281, 2560, 2561]),
+    (8, 1, 128, [256, 257, 768, 769, 2304, 2305, 2368, 2369])])
+def test_folds_of_many_ranges(dev, heads, kv_heads, head, depths):
+    errors = attention_errors(dev, _rope, heads, kv_heads, head, 16, depths)
     assert max(errors) < BAR, errors
 
 
