@@ -101,13 +101,33 @@ struct SplitAttn {
     };
 };
 
+// The keys of one CTA: start .. stop - 1 from the pages; the last range of a decode launch also has this step's own key, behind them.
+struct KeyRange {
+    int nsplit, start, stop;
+    bool owns_new;
+};
+__device__ __forceinline__ KeyRange key_range(const AttnArgs &a, int split, int pos) {
+    const int old = a.append != 0 ? pos : pos + 1;  // keys in the pages
+    KeyRange r;
+    r.nsplit = max(1, min(a.nsplit, (old + kKeysPerSplit - 1) / kKeysPerSplit));
+    const int chunk = (old + r.nsplit - 1) / r.nsplit;
+    r.start = min(old, split * chunk);
+    r.stop = min(old, r.start + chunk);
+    r.owns_new = a.append != 0 && split == r.nsplit - 1;
+    return r;
+}
+
 // The CTA's range once more, in scalar binary32, when an infinity or NaN showed in its output: a zero part of a query or
 // probability, or a row of the tile that holds no part, makes NaN of an infinite key or value, and so do parts of opposite signs.
 // Here, as in the reference, a score of -inf has no weight, an infinite value gives an infinite output, and a NaN score reaches the
 // output. Its speed matters to nobody: keys beyond 65504 do not occur in a model that works. Warp w takes every fourth key for
-// half of the heads; the results go to the merge area as the tiles' do. Ends with that area written, no barrier.
+// half of the heads; the results go to the merge area as the tiles' do. Ends with that area written, no barrier. A call, and one
+// that takes nothing from the caller's registers: in line it cost the launches that never get here 0.3 to 0.5 us in batches.
 template <int HD, int G>
-__device__ __forceinline__ void scalar_range(const AttnArgs &a, typename SplitAttn<HD, G>::Smem &sm, int b, int kvh, int pos, int slot, int start, int end) {
+__device__ __noinline__ void scalar_range(const AttnArgs &a, typename SplitAttn<HD, G>::Smem &sm) {
+    const int kvh = blockIdx.y, b = blockIdx.z, pos = a.positions[b], slot = a.slots[b];
+    const KeyRange keys = key_range(a, blockIdx.x, pos);
+    const int end = keys.stop + (keys.owns_new ? 1 : 0);
     constexpr int PAIRS = HD / 64;  // pairs of dimensions per lane
     const int lane = threadIdx.x & 31, kg = (threadIdx.x >> 5) % kGroups, half = (threadIdx.x >> 5) / kGroups;
     const int bt = a.kv.block_tokens, kv_dim = a.kv.kv_dim;
@@ -124,7 +144,7 @@ __device__ __forceinline__ void scalar_range(const AttnArgs &a, typename SplitAt
             o[i] = make_float2(0.f, 0.f);
         }
         float m = -INFINITY, l = 0.f;
-        for (int t = start + kg; t < end; t += kGroups) {
+        for (int t = keys.start + kg; t < end; t += kGroups) {
             const int64_t off = ((int64_t(table[t / bt]) * a.kv.layers + a.layer) * bt + t % bt) * kv_dim + int64_t(kvh) * HD;
             float2 v[PAIRS];
             float s = 0.f;
@@ -174,15 +194,13 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const __grid_co
     // were appended by the kernel ahead.
     if (!dec) pdl_wait();
     const int pos = on ? a.positions[b] : 0, slot = on ? a.slots[b] : 0;
-    const int old = dec ? pos : pos + 1;  // keys in the pages
-    const int nsplit = max(1, min(a.nsplit, (old + kKeysPerSplit - 1) / kKeysPerSplit));
+    const KeyRange keys = key_range(a, split, pos);
+    const int nsplit = keys.nsplit, start = keys.start, stop = keys.stop;
     if (!on || split >= nsplit) {
         if (dec) pdl_wait();
         return;
     }
-    const int chunk = (old + nsplit - 1) / nsplit;
-    const int start = min(old, split * chunk), stop = min(old, start + chunk);
-    const bool owns_new = dec && split == nsplit - 1;  // this step's own key and value: behind the last range
+    const bool owns_new = keys.owns_new;
     const int end = stop + (owns_new ? 1 : 0);
     const int bt = a.kv.block_tokens, kv_dim = a.kv.kv_dim;
     const int64_t block_stride = int64_t(a.kv.layers) * bt * kv_dim, in_layer = int64_t(a.layer) * bt * kv_dim + int64_t(kvh) * HD;
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_split_kernel(const __grid_co
     }
     // (a NaN score makes all outputs of its head NaN, so that they show it)
     if (__builtin_expect(__syncthreads_or(!(fabsf(all[0] + all[1]) < INFINITY)), 0)) {
-        scalar_range<HD, G>(a, sm, b, kvh, pos, slot, start, end);
+        scalar_range<HD, G>(a, sm);
         __syncthreads();
     }
     if (tid < G * kGroups) {  // four lanes per head: the groups' maxima and sums (one without keys weighs nothing)
