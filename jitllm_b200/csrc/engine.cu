@@ -893,8 +893,8 @@ int enqueue_rows_step(jl_ctx *ctx, int n, bool with_logits, bool advance, uint64
             if (!own_sequences && n >= tiled_min)
                 JL_LAUNCH(ctx, attention_prompt_launch(a, n, ctx->stream, ctx->use_pdl), "prompt attention");
             else if (own_sequences && n >= 4 && n * ctx->l_kv_heads >= ctx->batch_attn_min_pairs)
-                // enough (row, KV head) pairs to fill the GPU with one CTA each: the tensor-core walk; narrower
-                // batches keep the kernel that splits a sequence's keys over a cluster of CTAs
+                // enough (row, KV head) pairs to fill the GPU with one CTA each; narrower batches take the kernel that
+                // splits a sequence's keys over CTAs
                 JL_LAUNCH(ctx, attention_batch_launch(a, n, ctx->stream, ctx->use_pdl), "batch attention");
             else
                 JL_LAUNCH(ctx, attention_launch(a, n, ctx->stream, ctx->use_pdl), "attention");
@@ -1223,8 +1223,12 @@ int32_t jl_init(int32_t device_id, jl_ctx **out) {
     ctx->use_graph = env_flag("JITLLM_B200_GRAPH", true);
     ctx->use_pdl = env_flag("JITLLM_B200_PDL", true);
     {
-        // enough (row, KV head) pairs to give most SMs a CTA of their own: the tensor-core walk of
-        // attention_batch_launch; narrower batches keep the kernel that splits a sequence's keys over a cluster
+        // (row, KV head) pairs from which one CTA per pair (attention_batch_launch) takes over from ranges of keys
+        // (attention_launch). Below three quarters of the SMs, pairs alone leave the GPU idle: a step of eight 8B layers with 12 rows
+        // (96 pairs) takes 819 / 893 / 1085 / 1630 us at 100 / 500 / 1500 / 4000 keys with a CTA per pair, 812 / 856 / 996 / 1356
+        // with ranges. From 14 rows to 18 the two differ by 1.5 % at most (14 rows 830 / 903 / 1098 / 1635 and 823 / 895 / 1103 / 1635).
+        // From 20 on ranges need a second wave (20 rows 872 / 951 / 1152 and 859 / 1014 / 1450). With head size 64: 12 rows 419 / 489 / 653
+        // and 430 / 468 / 566, 14 rows 423 / 495 / 659 and 434 / 484 / 630, 20 rows 480 / 553 / 727 and 484 / 600 / 892.
         const char *v = getenv("JITLLM_B200_BATCH_ATTN_MIN_PAIRS");
         ctx->batch_attn_min_pairs = v ? atoi(v) : (3 * ctx->sm_count) / 4;
     }
