@@ -347,10 +347,9 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4],
 // own (cp.async, two groups of sixteen ahead) and keeps its own running maximum, sum and output, merged at the end.
 // Nothing but the pages' arrival should bound this kernel, so the instructions beside the products are few: the
 // sixteen keys of a group share a page whenever the page size is a multiple of sixteen, and then one page lookup and
-// one pointer serve all of a lane's copies of the group; no barrier of the CTA stands between two groups. (With
-// tiles of 64 keys staged by the whole CTA, every key divided by the page size for its own address and two barriers
-// a tile, a step of the 8B shape took 4519 us with 32 rows of 256-768 keys, now 4210: 9.7 us less in each of 32 launches;
-// with 64 rows of 210-630 keys the gain is the same.)
+// one pointer serve all of a lane's copies of the group; no barrier of the CTA stands between two groups. A step of the 8B
+// shape with 32 rows of 256-768 keys takes 4210 us this way; with tiles of 64 keys staged by the whole CTA, an address division
+// for every key and two barriers a tile it is 4519 (9.7 us more in each of 32 launches).
 // The step's own key and value (rotated, rounded to binary16 as the append does) are written to the page and
 // dropped into the staged group by the warp that holds it, so nothing else has to run before it.
 // Arithmetic: inference/op/CpuOperations.java:94-235, as attn_split.cu.
